@@ -525,7 +525,9 @@ int sunset_calc_gradient(SunsetHandle *sh, const double *phi, double *grad, int 
     if (flags == SUNSET_PTR_DEVICE) {
         std::vector<double> inter(2 * (size_t)n);
         for (int r = 0; r < n; r++) { inter[2 * r] = hx[r]; inter[2 * r + 1] = hy[r]; }
-        SUNSET_CUDA(H, cudaMemcpy(grad, inter.data(), inter.size() * sizeof(double), cudaMemcpyHostToDevice));
+        SUNSET_CUDA(H, cudaMemcpyAsync(grad, inter.data(), inter.size() * sizeof(double), cudaMemcpyHostToDevice,
+                                       H->stream));
+        SUNSET_CUDA(H, cudaStreamSynchronize(H->stream));
     } else {
         for (int r = 0; r < n; r++) { grad[2 * r] = hx[r]; grad[2 * r + 1] = hy[r]; }
     }
@@ -856,8 +858,8 @@ int sunset_set_lengths(SunsetHandle *sh, const double *h, const double *h_small)
         hsv[i] = h_small[r];
         H->hmax = std::max(H->hmax, h[r]);
     }
-    SUNSET_CUDA(H, cudaMemcpy(H->h, hv.data(), n * sizeof(double), cudaMemcpyHostToDevice));
-    SUNSET_CUDA(H, cudaMemcpy(H->hs, hsv.data(), n * sizeof(double), cudaMemcpyHostToDevice));
+    SUNSET_CUDA(H, cudaMemcpyAsync(H->h, hv.data(), n * sizeof(double), cudaMemcpyHostToDevice, H->stream));
+    SUNSET_CUDA(H, cudaMemcpyAsync(H->hs, hsv.data(), n * sizeof(double), cudaMemcpyHostToDevice, H->stream));
     return 0;
 }
 
@@ -1000,7 +1002,7 @@ int sunset_set_restart(SunsetHandle *sh, const double *columns, const double *he
     sc.emax_n = header[6];
     sc.emax_nm1 = header[7];
     sc.dt = header[8];
-    SUNSET_CUDA(H, cudaMemcpy(H->dsc, &sc, sizeof(sc), cudaMemcpyHostToDevice));
+    SUNSET_CUDA(H, cudaMemcpyAsync(H->dsc, &sc, sizeof(sc), cudaMemcpyHostToDevice, H->stream));
     return 0;
 }
 
@@ -1032,7 +1034,7 @@ int sunset_set_flow_control(SunsetHandle *sh, const double *in) {
     sc.eflow_nm1 = in[0];
     sc.sum_eflow = in[1];
     sc.df = in[2];
-    SUNSET_CUDA(H, cudaMemcpy(H->dsc, &sc, sizeof(sc), cudaMemcpyHostToDevice));
+    SUNSET_CUDA(H, cudaMemcpyAsync(H->dsc, &sc, sizeof(sc), cudaMemcpyHostToDevice, H->stream));
     return 0;
 }
 

@@ -629,9 +629,9 @@ int build_halos(Handle *H) {
     for (int t = 0; t < nt; t++) std::copy(halos[t].begin(), halos[t].end(), hall.begin() + hptr[t]);
     if (dalloc(H, &H->halo_ptr, nt + 1) || dalloc(H, &H->halo, hall.size()) || dalloc(H, &H->lloc, L))
         return SUNSET_ERR_NOMEM;
-    SUNSET_CUDA(H, cudaMemcpy(H->halo_ptr, hptr.data(), hptr.size() * sizeof(int), cudaMemcpyHostToDevice));
-    SUNSET_CUDA(H, cudaMemcpy(H->halo, hall.data(), hall.size() * sizeof(int), cudaMemcpyHostToDevice));
-    SUNSET_CUDA(H, cudaMemcpy(H->lloc, loc.data(), L * sizeof(uint16_t), cudaMemcpyHostToDevice));
+    SUNSET_CUDA(H, cudaMemcpyAsync(H->halo_ptr, hptr.data(), hptr.size() * sizeof(int), cudaMemcpyHostToDevice, H->stream));
+    SUNSET_CUDA(H, cudaMemcpyAsync(H->halo, hall.data(), hall.size() * sizeof(int), cudaMemcpyHostToDevice, H->stream));
+    SUNSET_CUDA(H, cudaMemcpyAsync(H->lloc, loc.data(), L * sizeof(uint16_t), cudaMemcpyHostToDevice, H->stream));
     H->ntiles = nt;
     H->halo_max = hmax;
     return 0;
