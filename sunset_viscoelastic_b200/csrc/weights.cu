@@ -1,14 +1,15 @@
 // weights.cu -- LABFM weight construction on the device (labf.F90, svdlib.F90, rbfs.F90).
 //
-// One warp builds the weights of one node: it assembles the moment matrix
-// A = sum_k X(r_k/h) [W(r_k/h) H(r_k/h)]^T (monomials X, Hermite ABFs H, Wendland C2 W)
-// in shared memory, factors it with the reference's Golub-Kahan-Reinsch SVD and applies
-// the factorisation to each right-hand side.  The SVD is the reference's algorithm with
-// its serial recurrences kept serial: lanes split only loops whose iterations are
-// independent (columns of a Householder update, rows of a Givens rotation), and every
-// dot product is summed by one lane in the reference's order.  With -fmad=false each
-// operation then rounds exactly as the reference's does, so the factorisation - and the
-// weights - are those of the CPU restatement bit for bit.
+// The weights of a node: its moment matrix
+// A = sum_k X(r_k/h) [W(r_k/h) H(r_k/h)]^T (monomials X, Hermite ABFs H, Wendland C2 W),
+// factored with the reference's Golub-Kahan-Reinsch SVD, and the factorisation applied to each
+// right-hand side.  The SVD is the reference's algorithm with its serial recurrences kept
+// serial: threads split only loops whose iterations are independent (columns of a Householder
+// update, rows of a Givens rotation), and every dot product is summed by one thread in the
+// reference's order.  With -fmad=false each operation then rounds exactly as the
+// reference's does, so the factorisation - and the weights - are those of the CPU
+// restatement bit for bit.  The weight build takes three kernels (below); the stencil
+// adaptation and the boundary operators factor on one warp (svd_factor_warp).
 //
 // The five SVDs of identical matrix copies in labf.F90:157-180 become one factorisation
 // applied to five right-hand sides; the filter matrix (labf.F90:258-303) is the same
@@ -415,138 +416,640 @@ __device__ void assemble(const WArgs &a, int i, int cnt, double hh, double *U, i
     __syncwarp();
 }
 
-// labf.F90:125-148: keep the first m unknowns.
-template <int N>
-__device__ void drop_order(double *U, int ld, int m, int lane) {
-    __syncwarp();
-    for (int e = lane; e < N * N; e += 32) {
-        int i1 = e % N, i2 = e / N;
-        if (i2 >= m || i1 >= m) U[i2 * ld + i1] = (i1 == i2) ? 1.0 : 0.0;
-    }
-    __syncwarp();
+// ---------------------------------------------------------------------------------------
+// The weight build in three kernels over batches of nodes.
+//
+// One warp doing everything for a node (assembly, SVD, solves) spent nine tenths of its time
+// in the QR iteration's scalar recurrence (two hypotenuses, three divisions and a reciprocal a
+// rotation, each waiting for the one before) with the node's two matrices parked in shared
+// memory, so that six warps a SM filled it: 1.94 s for 1,048,576 nodes at order 8, 26 % of
+// the issue slots used.  That recurrence reads only the bidiagonal, never the matrices, so
+// it is taken out of the middle:
+//   k_moment_bidiag  a block a node: moment matrix (accumulators in registers, a column a
+//                    thread), Householder bidiagonalisation and both accumulations;
+//   k_bidiag_qr      a thread a node: the QR iteration on the bidiagonal, recording its
+//                    rotations;
+//   k_weights_apply  a warp a node: the rotations replayed on the rows that the solves read,
+//                    the solves and the link weights.
+// A rotation acts on each row of U and V by itself, and the right-hand sides are unit vectors
+// (or the few entries of the hyperviscous operator), so of U only the four to ten rows that
+// meet a nonzero entry are replayed.  Every sum, rotation and solve keeps its order and
+// rounding, so the weights stay the reference's bit for bit.
+//
+// A node whose rotations do not fit its record stops before the sweep that would not fit, and
+// the last two kernels run again until every node is done.
+//
+// 1,048,576 nodes at order 8: 1943 -> 515 ms (262,144: 99 + 7 + 18 ms in the three kernels).
+// ---------------------------------------------------------------------------------------
+constexpr int kUrows = 10;  // rows of U the solves read: 0, 1, 2, 4 and up to six of the filter's
+
+// Entry c of the hyperviscous right-hand side (labf.F90:325-388): its row, with its value.
+__host__ __device__ __forceinline__ int hyp_entry(int order, int c, double *v) {
+    const int half = order <= 5 ? 2 : order <= 7 ? 3 : order <= 9 ? 4 : 5;
+    if (c > half) return -1;
+    double b = 1.0;  // the binomial coefficient of half over c
+    for (int k = 1; k <= c; k++) b = b * (double)(half - k + 1) / (double)k;
+    *v = (half & 1) ? b : -b;
+    const int d = 2 * half;
+    return (d * d + d) / 2 - 1 + 2 * c;  // unknowns of degree d start at d (d + 1) / 2 - 1
 }
 
-__device__ void hyp_rhs(int order, double *b, int n, int lane) {
-    __syncwarp();
-    for (int m = lane; m < n; m += 32) b[m] = 0.0;
-    __syncwarp();
-    if (lane == 0) {
-        if (order <= 5) { b[9] = -1.0; b[11] = -2.0; b[13] = -1.0; }
-        else if (order <= 7) { b[20] = 1.0; b[22] = 3.0; b[24] = 3.0; b[26] = 1.0; }
-        else if (order <= 9) { b[35] = -1.0; b[37] = -4.0; b[39] = -6.0; b[41] = -4.0; b[43] = -1.0; }
-        else { b[54] = 1.0; b[56] = 5.0; b[58] = 10.0; b[60] = 10.0; b[62] = 5.0; b[64] = 1.0; }
-    }
-    __syncwarp();
+// Order of a node's hyperviscous operator (labf.F90:305-323): reduced next to walls.
+__device__ __forceinline__ int filter_order(int forder, int t) {
+    int o = forder;
+    if (forder >= 7 && (t == 998 || t < 0)) o = 6;
+    if (forder >= 5 && t == -1) o = 4;
+    return o;
 }
 
+// What the three kernels share for one batch.  Arrays of [..][batch] are indexed by the item
+// last, so that a thread an item reads them coalesced; a rotation is four doubles (cosine and
+// sine on V, then on U) in the item's own record.
+struct SvdBatch {
+    int n_items, batch, cap;  // items; their capacity; rotations a record holds
+    const int *item;          // the node of each item
+    int pass;                 // 0: derivative matrix (and the filter where it is the same one), 1: filter
+    double *W, *rv1;          // [n + 1][batch], 1-based
+    double *anorm;            // [batch]
+    int2 *state;              // singular value and sweep to go on from; {0, 0}: done, {-1, 0}: no convergence
+    int *nrec;                // record entries of the last k_bidiag_qr; -1: done before it
+    double *U, *V;            // [batch][kUrows][n] and [batch][n][n] (column by column)
+    double4 *rec;             // [batch][cap]
+    int *left;                // items not done yet
+};
+
+__host__ __device__ constexpr int bidiag_threads(int order) { return (nsz(order) + 31) / 32 * 32; }
+constexpr int kAsmLinks = 32;  // links whose monomials are staged at once
+// Doubles of shared memory of k_moment_bidiag: U, V and three vectors; while the moment
+// matrix is assembled, U's and V's place holds the chunk's powers, Hermite polynomials and
+// monomials.
 template <int ORDER>
-__host__ __device__ constexpr int smem_doubles() {
-    return 2 * nsz(ORDER) * (nsz(ORDER) | 1) + 3 * (nsz(ORDER) + 2) + 7 * nsz(ORDER);
+__host__ __device__ constexpr int bidiag_doubles() {
+    constexpr int n = nsz(ORDER), mats = 2 * n * (n | 1), stage = kAsmLinks * (4 * (ORDER + 1) + 1 + n);
+    return (mats > stage ? mats : stage) + 2 * (n + 2);
 }
 
+// Whether the filter's moment matrix is the derivative one (labf.F90:258-303).
+__device__ __forceinline__ bool same_matrix(const WArgs &a, int i, int t) {
+    return a.h[i] == a.hs[i] && a.cnt[i] == a.cnt_small[i] && a.forder == a.morder && t != -2;
+}
+
+// Items of the two passes: every node but the boundary nodes, and those whose filter matrix
+// is another one.
+__global__ void k_weight_items(WArgs a, int *item0, int *item1, int *count) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= a.npfb) return;
+    const int t = a.ntype[i];
+    if (!(t < 0 || t == 999 || t == 998)) return;  // boundary nodes: labf.F90:505-1039
+    item0[atomicAdd(&count[0], 1)] = i;
+    if (!same_matrix(a, i, t)) item1[atomicAdd(&count[1], 1)] = i;
+}
+
+// Moment matrix (labf.F90:88-148 or 258-303) and svdlib.F90:37-171 of one node a block.
+// Bound: the FP64 sums in the reference's serial order (a column's dot product is one chain),
+// seven blocks of two warps a SM at order 8 (32 KB of shared memory each).
 template <int ORDER>
-__global__ void k_labf_weights(WArgs a) {
-    constexpr int n = nsz(ORDER);
-    constexpr int ld = n | 1;
+__global__ void __launch_bounds__(bidiag_threads(ORDER)) k_moment_bidiag(WArgs a, SvdBatch B) {
+    constexpr int n = nsz(ORDER), ld = n | 1, T = bidiag_threads(ORDER);
     extern __shared__ double smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-    double *U = smem + warp * smem_doubles<ORDER>();
-    double *V = U + n * ld, *W = V + n * ld, *rv1 = W + (n + 2), *tmp = rv1 + (n + 2);
-    double *X = tmp + (n + 2), *G = X + n, *bx = G + n, *by = bx + n, *bxx = by + n, *byy = bxx + n, *bh = byy + n;
-    for (int i = blockIdx.x * wpb + warp; i < a.npfb; i += gridDim.x * wpb) {
-        const int t = a.ntype[i];
-        if (!(t < 0 || t == 999 || t == 998)) continue;  // boundary nodes: labf.F90:505-1039
-        const int cnt = a.cnt[i], cs = a.cnt_small[i];
-        double hh = a.hs[i];
-        // ---- derivative weights, labf.F90:80-215 ----
-        assemble<ORDER>(a, i, cs, hh, U, ld, X, G, lane);
-        if (a.morder >= 7 && (t == 998 || t < 0)) drop_order<n>(U, ld, 27, lane);
-        if (a.morder >= 5 && (t == -1 || t == -2)) drop_order<n>(U, ld, 14, lane);
-        if (svd_factor_warp<n>(U, V, W, rv1, ld, lane, a.maxits > 0 ? a.maxits : 30)) {
-            if (lane == 0) atomicExch(a.err, i + 1);
-            continue;
+    const int it = blockIdx.x, tid = threadIdx.x;
+    const int i0 = B.item[it], t = a.ntype[i0];
+    double *U = smem, *V = U + n * ld;
+    double *rv1 = smem + bidiag_doubles<ORDER>() - 2 * (n + 2), *W = rv1 + (n + 2);
+    auto sync = [] {
+        if constexpr (T == 32) __syncwarp();
+        else __syncthreads();
+    };
+    const double hh = B.pass ? a.h[i0] : a.hs[i0];
+    const int cnt = B.pass ? a.cnt[i0] : a.cnt_small[i0];
+    {
+        // the thread's unknown: exponents and 1 / (p! q!) of its monomial (see monomial())
+        const int m = tid < n ? tid : 0;
+        const int pm = p_of(m), qm = q_of(m);
+        const double den = fact(pm) * fact(qm), inv = 1.0 / den;
+        double acc[n];
+#pragma unroll
+        for (int r = 0; r < n; r++) acc[r] = 0.0;
+        constexpr int P = ORDER + 1;
+        double *xp = smem, *yp = xp + kAsmLinks * P, *hx = yp + kAsmLinks * P, *hy = hx + kAsmLinks * P;
+        double *ker = hy + kAsmLinks * P, *X = ker + kAsmLinks;
+        const double xi = a.px[i0], yi = a.py[i0];
+        for (int k0 = 0; k0 < cnt; k0 += kAsmLinks) {
+            const int nk = min(kAsmLinks, cnt - k0);
+            sync();
+            if (tid < nk) {
+                const int p = a.lpt[sell_off(a.slice_ptr, i0, k0 + tid)];
+                const double x = -(xi - a.px[p]), y = -(yi - a.py[p]);
+                const double rad = sqrt(x * x + y * y) / hh;
+                ker[tid] = wab(rad, a.h2);
+                const double xx = x / hh, yy = y / hh;
+                double px = xx, py = yy;
+                xp[tid] = yp[tid] = 1.0;
+#pragma unroll
+                for (int d = 1; d <= ORDER; d++) {
+                    xp[d * kAsmLinks + tid] = px;
+                    yp[d * kAsmLinks + tid] = py;
+                    px = px * xx;
+                    py = py * yy;
+                }
+#pragma unroll
+                for (int d = 0; d <= ORDER; d++) {
+                    hx[d * kAsmLinks + tid] = hermite(d, xx);
+                    hy[d * kAsmLinks + tid] = hermite(d, yy);
+                }
+            }
+            sync();
+            if (tid < n)
+                for (int k = 0; k < nk; k++) {
+                    const double xv = xp[pm * kAsmLinks + k], yv = yp[qm * kAsmLinks + k];
+                    double v;
+                    if (den == 1.0) v = pm == 0 ? yv : qm == 0 ? xv : xv * yv;
+                    else v = qm == 0 ? inv * xv : pm == 0 ? inv * yv : (inv * xv) * yv;
+                    X[k * n + tid] = v;
+                }
+            sync();
+            for (int k = 0; k < nk; k++) {
+                const double hxv = hx[pm * kAsmLinks + k], hyv = hy[qm * kAsmLinks + k];
+                const double g = (qm == 0 ? hxv : pm == 0 ? hyv : hxv * hyv) * ker[k];
+#pragma unroll
+                for (int r = 0; r < n; r++) acc[r] = acc[r] + X[k * n + r] * g;
+            }
         }
-        double cond_d = 0.0;
-        if (lane == 0) cond_d = svd_cond<n>(W);
-        if (lane == 0 && a.cond_d) a.cond_d[i] = cond_d;
-        for (int m = lane; m < n; m += 32) {
-            bx[m] = (m == 0) ? 1.0 : 0.0;
-            by[m] = (m == 1) ? 1.0 : 0.0;
-            bxx[m] = (m == 2) ? 1.0 : 0.0;
-            byy[m] = (m == 4) ? 1.0 : 0.0;
+        sync();
+        // labf.F90:125-148, 305-323: next to walls only the first unknowns are kept
+        int keep = n;
+        if (B.pass == 0) {
+            if (a.morder >= 7 && (t == 998 || t < 0)) keep = min(keep, 27);
+            if (a.morder >= 5 && (t == -1 || t == -2)) keep = min(keep, 14);
+        } else {
+            if (a.forder >= 7 && (t == 998 || t < 0)) keep = min(keep, 27);
+            if (a.forder >= 5 && t == -1) keep = min(keep, 14);
         }
-        svd_apply_warp<n>(U, V, W, tmp, bx, ld, lane);
-        svd_apply_warp<n>(U, V, W, tmp, by, ld, lane);
-        svd_apply_warp<n>(U, V, W, tmp, bxx, ld, lane);
-        svd_apply_warp<n>(U, V, W, tmp, byy, ld, lane);
-        for (int m = lane; m < n; m += 32) bxx[m] = bxx[m] + byy[m];  // bvecxx + bvecyy
+        if (tid < n) {
+#pragma unroll
+            for (int r = 0; r < n; r++) U[tid * ld + r] = (tid >= keep || r >= keep) ? (r == tid ? 1.0 : 0.0) : acc[r];
+        }
+        sync();
+    }
+#define UM(i, j) U[((j) - 1) * ld + ((i) - 1)]
+#define VM(i, j) V[((j) - 1) * ld + ((i) - 1)]
+    // svdlib.F90:37-113.  The scalars are computed by every thread alike; the pivot f - g stays in
+    // a register until the column (row) is scaled back.
+    double anorm = 0.0, g = 0.0, scale = 0.0;
+    int l = 1;
+    const int me = tid + 1;  // the thread's column, row or entry, 1-based
+    for (int i = 1; i <= n; i++) {
+        l = i + 1;
+        const double ri = scale * g;
+        if (tid == 0) rv1[i] = ri;
+        g = 0.0;
+        double s = 0.0;
+        scale = 0.0;
+#pragma unroll 4
+        for (int k = i; k <= n; k++) scale = scale + fabs(UM(k, i));
+        if (scale != 0.0) {
+            sync();
+            if (me >= i && me <= n) UM(me, i) = UM(me, i) / scale;
+            sync();
+#pragma unroll 4
+            for (int k = i; k <= n; k++) s = s + UM(k, i) * UM(k, i);
+            const double f = UM(i, i);
+            g = -copysign(sqrt(s), f);
+            const double h = f * g - s, piv = f - g;
+            if (me >= l && me <= n) {
+                double sj = 0.0;
+                sj = sj + piv * UM(i, me);
+#pragma unroll 4
+                for (int k = l; k <= n; k++) sj = sj + UM(k, i) * UM(k, me);
+                const double fj = sj / h;
+                UM(i, me) = UM(i, me) + fj * piv;
+#pragma unroll 4
+                for (int k = l; k <= n; k++) UM(k, me) = UM(k, me) + fj * UM(k, i);
+            }
+            sync();
+            if (me >= i && me <= n) UM(me, i) = scale * (me == i ? piv : UM(me, i));
+        }
+        const double wi = scale * g;
+        if (tid == 0) W[i] = wi;
+        g = 0.0; s = 0.0; scale = 0.0;
+#pragma unroll 4
+        for (int k = l; k <= n; k++) scale = scale + fabs(UM(i, k));
+        if (scale != 0.0) {
+            sync();
+            if (me >= l && me <= n) UM(i, me) = UM(i, me) / scale;
+            sync();
+#pragma unroll 4
+            for (int k = l; k <= n; k++) s = s + UM(i, k) * UM(i, k);
+            const double f = UM(i, l);
+            g = -copysign(sqrt(s), f);
+            const double h = f * g - s, piv = f - g;
+            if (me >= l && me <= n) rv1[me] = (me == l ? piv : UM(i, me)) / h;
+            sync();
+            if (me >= l && me <= n) {
+                double sj = 0.0;
+                sj = sj + UM(me, l) * piv;
+#pragma unroll 4
+                for (int k = l + 1; k <= n; k++) sj = sj + UM(me, k) * UM(i, k);
+#pragma unroll 4
+                for (int k = l; k <= n; k++) UM(me, k) = UM(me, k) + sj * rv1[k];
+            }
+            sync();
+            if (me >= l && me <= n) UM(i, me) = scale * (me == l ? piv : UM(i, me));
+        }
+        sync();
+        const double tn = fabs(wi) + fabs(ri);
+        anorm = (tn > anorm) ? tn : anorm;
+    }
+    // right-hand transformations, svdlib.F90:115-141
+    g = 0.0;
+    for (int i = n; i >= 1; i--) {
+        if (i < n) {
+            if (g != 0.0) {
+                if (me >= l && me <= n) VM(me, i) = (UM(i, me) / UM(i, l)) / g;
+                sync();
+                if (me >= l && me <= n) {
+                    double sj = 0.0;
+#pragma unroll 4
+                    for (int k = l; k <= n; k++) sj = sj + UM(i, k) * VM(k, me);
+#pragma unroll 4
+                    for (int k = l; k <= n; k++) VM(k, me) = VM(k, me) + sj * VM(k, i);
+                }
+                sync();
+            }
+            if (me >= l && me <= n) { VM(i, me) = 0.0; VM(me, i) = 0.0; }
+        }
+        if (tid == 0) VM(i, i) = 1.0;
+        sync();
+        g = rv1[i];
+        l = i;
+    }
+    // left-hand transformations, svdlib.F90:143-171
+    for (int i = n; i >= 1; i--) {
+        l = i + 1;
+        g = W[i];
+        if (me >= l && me <= n) UM(i, me) = 0.0;  // read back by the same thread only
+        const double pii = UM(i, i);
+        if (g != 0.0) {
+            g = 1.0 / g;
+            if (me >= l && me <= n) {
+                double sj = 0.0;
+#pragma unroll 4
+                for (int k = l; k <= n; k++) sj = sj + UM(k, i) * UM(k, me);
+                const double fj = (sj / pii) * g;
+                UM(i, me) = UM(i, me) + fj * pii;
+#pragma unroll 4
+                for (int k = l; k <= n; k++) UM(k, me) = UM(k, me) + fj * UM(k, i);
+            }
+            sync();
+            if (me >= i && me <= n) UM(me, i) = me == i ? pii * g + 1.0 : UM(me, i) * g;
+        } else {
+            sync();
+            if (me >= i && me <= n) UM(me, i) = me == i ? 0.0 + 1.0 : 0.0;
+        }
+        sync();
+    }
+    // the rows of U that the solves read, V, and the bidiagonal
+    const int fo = filter_order(a.forder, t);
+    for (int e = tid; e < kUrows * n; e += T) {
+        const int r = e / n, c = e % n;
+        double dummy;
+        int row = r < 3 ? r : 4;
+        if (r >= 4) row = hyp_entry(fo, r - 4, &dummy);
+        B.U[(size_t)it * kUrows * n + e] = row >= 0 && row < n ? U[c * ld + row] : 0.0;
+    }
+    for (int e = tid; e < n * n; e += T) B.V[(size_t)it * n * n + e] = V[(e / n) * ld + e % n];
+    if (me <= n) {
+        B.W[(size_t)me * B.batch + it] = W[me];
+        B.rv1[(size_t)me * B.batch + it] = rv1[me];
+    }
+    if (tid == 0) {
+        B.anorm[it] = anorm;
+        B.state[it] = make_int2(n, 1);
+    }
+#undef UM
+#undef VM
+}
+
+// What a record entry's header says the entries after it are.
+enum { kRecSweep = 0, kRecCancel = 1, kRecNegate = 2 };
+__device__ __forceinline__ double4 rec_header(int kind, int col, int count) {
+    return make_double4(__hiloint2double(kind, col), __hiloint2double(0, count), 0.0, 0.0);
+}
+
+constexpr int kQrThreads = 32;
+
+// svdlib.F90:173-278 on the bidiagonal alone, one thread an item.  The item's record gets, for
+// each sweep, a header (kind, first column, entries) and the rotations.  Bound: the latency of
+// the recurrence (about 700 cycles a rotation), hidden by as many items as the batch has.
+template <int ORDER>
+__global__ void __launch_bounds__(kQrThreads) k_bidiag_qr(SvdBatch B, int maxits) {
+    constexpr int n = nsz(ORDER);
+    extern __shared__ double smem[];
+    const int it = blockIdx.x * kQrThreads + threadIdx.x;
+    if (it >= B.n_items) return;
+    const int2 st = B.state[it];
+    if (st.x <= 0) {
+        B.nrec[it] = -1;
+        return;
+    }
+    double *Ws = smem + threadIdx.x, *Rs = Ws + (n + 1) * kQrThreads;
+#define WQ(j) Ws[(j) * kQrThreads]
+#define RQ(j) Rs[(j) * kQrThreads]
+    for (int j = 1; j <= n; j++) {
+        WQ(j) = B.W[(size_t)j * B.batch + it];
+        RQ(j) = B.rv1[(size_t)j * B.batch + it];
+    }
+    const double anorm = B.anorm[it];
+    double4 *rec = B.rec + (size_t)it * B.cap;
+    int pos = 0;
+    int2 next = make_int2(0, 0);
+    int its0 = st.y;
+    for (int k = st.x; k >= 1; k--) {
+        bool stop = false;
+        for (int its = its0; its <= 30; its++) {
+            if (pos + 2 * n + 4 > B.cap) {  // a sweep and a cancellation at most before the next look
+                next = make_int2(k, its);
+                stop = true;
+                break;
+            }
+            bool to2000 = false;
+            int l, nm = 1;
+            for (l = k; l >= 1; l--) {
+                nm = l - 1;
+                if ((fabs(RQ(l)) + anorm) == anorm) { to2000 = true; break; }
+                if ((fabs(WQ(nm)) + anorm) == anorm) break;
+            }
+            if (l < 1) {  // no split found: only a NaN in the bidiagonal gets here
+                next = make_int2(-1, 0);
+                stop = true;
+                break;
+            }
+            double c, s, f, g, h, x, y, z;
+            if (!to2000) {
+                const int at = pos++;
+                int m = 0;
+                c = 0.0; s = 1.0;
+                for (int i = l; i <= k; i++) {
+                    const double r = RQ(i);
+                    f = s * r;
+                    RQ(i) = c * r;
+                    if ((fabs(f) + anorm) == anorm) break;
+                    g = WQ(i);
+                    h = nr_hypot(f, g);
+                    WQ(i) = h;
+                    h = 1.0 / h;
+                    c = (g * h);
+                    s = -(f * h);
+                    rec[pos++] = make_double4(0.0, 0.0, c, s);
+                    m++;
+                }
+                rec[at] = rec_header(kRecCancel, l, m);
+            }
+            z = WQ(k);
+            if (l == k) {
+                if (z < 0.0) {
+                    WQ(k) = -z;
+                    rec[pos++] = rec_header(kRecNegate, k, 0);
+                }
+                break;
+            }
+            if (its >= maxits) {
+                next = make_int2(-1, 0);
+                stop = true;
+                break;
+            }
+            x = WQ(l);
+            nm = k - 1;
+            y = WQ(nm);
+            g = RQ(nm);
+            h = RQ(k);
+            f = ((y - z) * (y + z) + (g - h) * (g + h)) / ((2.0 * h) * y);
+            g = nr_hypot(f, 1.0);
+            f = ((x - z) * (x + z) + h * ((y / (f + copysign(g, f))) - h)) / x;
+            c = 1.0; s = 1.0;
+            rec[pos++] = rec_header(kRecSweep, l, nm - l + 1);
+            for (int j = l; j <= nm; j++) {
+                const int i = j + 1;
+                g = RQ(i);
+                y = WQ(i);
+                h = s * g;
+                g = c * g;
+                z = nr_hypot(f, h);
+                RQ(j) = z;
+                c = f / z;
+                s = h / z;
+                const double c1 = c, s1 = s;
+                f = (x * c) + (g * s);
+                g = -(x * s) + (g * c);
+                h = y * s;
+                y = y * c;
+                z = nr_hypot(f, h);
+                WQ(j) = z;
+                if (z != 0.0) {
+                    z = 1.0 / z;
+                    c = f * z;
+                    s = h * z;
+                }
+                f = (c * g) + (s * y);
+                x = -(s * g) + (c * y);
+                rec[pos++] = make_double4(c1, s1, c, s);
+            }
+            RQ(l) = 0.0;
+            RQ(k) = f;
+            WQ(k) = x;
+        }
+        if (stop) break;
+        its0 = 1;
+    }
+    for (int j = 1; j <= n; j++) {
+        B.W[(size_t)j * B.batch + it] = WQ(j);
+        B.rv1[(size_t)j * B.batch + it] = RQ(j);
+    }
+    B.state[it] = next;
+    B.nrec[it] = pos;
+    if (next.x > 0) atomicAdd(B.left, 1);
+#undef WQ
+#undef RQ
+}
+
+constexpr int kApplyWarps = 1;  // items a block of k_weights_apply (one warp each)
+template <int ORDER>
+__host__ __device__ constexpr int apply_doubles() {
+    // rows [n + kUrows][n | 1], two staged halves of 32 record entries, W, one solve, five results
+    return ((nsz(ORDER) + kUrows) * (nsz(ORDER) | 1) + 2 * 32 * 4 + (nsz(ORDER) + 2) + 6 * nsz(ORDER) + 3) & ~3;
+}
+
+// The recorded rotations replayed on the item's rows (lanes take rows; a sweep's rotation j acts
+// on columns j and j + 1, so the second column stays in a register for the next one), then,
+// once the item is done, svdlib.F90:279-303 for each right-hand side and the weights of its
+// links (labf.F90:157-231, 325-388).  Bound: issue slots and FP64 (12 multiplies and adds and
+// 2 shared loads and stores a rotation and warp).
+template <int ORDER>
+__global__ void __launch_bounds__(kApplyWarps * 32) k_weights_apply(WArgs a, SvdBatch B) {
+    constexpr int n = nsz(ORDER), ld = n | 1, rows = n + kUrows, SL = (rows + 31) / 32;
+    extern __shared__ __align__(32) double smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int it = blockIdx.x * kApplyWarps + warp;
+    if (it >= B.n_items) return;
+    const int2 st = B.state[it];
+    const int nrec = B.nrec[it];
+    if (nrec < 0) return;  // done in an earlier round
+    double *stage = smem + (size_t)warp * apply_doubles<ORDER>();  // first, for its alignment
+    double *R = stage + 2 * 32 * 4, *W = R + rows * ld, *tmp = W + (n + 2), *bx = tmp + n, *by = bx + n,
+           *bxx = by + n, *byy = bxx + n, *bh = byy + n;
+    const int i = B.item[it], t = a.ntype[i];
+    if (st.x < 0) {
+        if (lane == 0) atomicExch(a.err, i + 1);
+        return;
+    }
+    double *Vg = B.V + (size_t)it * n * n, *Ug = B.U + (size_t)it * kUrows * n;
+    for (int e = lane; e < n * n; e += 32) R[(e % n) * ld + e / n] = Vg[e];
+    for (int e = lane; e < kUrows * n; e += 32) R[(n + e / n) * ld + e % n] = Ug[e];
+    const double4 *rec = B.rec + (size_t)it * B.cap;
+    double4 pre = lane < nrec ? rec[lane] : make_double4(0, 0, 0, 0);
+    int e = 0;
+    // entry e of the record: 32 at a time come in ahead of their use
+    auto fetch = [&]() -> double4 {
+        if ((e & 31) == 0) {
+            __syncwarp();
+            reinterpret_cast<double4 *>(stage)[(e & 32) + lane] = pre;
+            if (e + 32 + lane < nrec) pre = rec[e + 32 + lane];
+            __syncwarp();
+        }
+        const double4 v = reinterpret_cast<const double4 *>(stage)[e & 63];
+        e++;
+        return v;
+    };
+    double *row[SL];
+    bool isu[SL], live[SL];
+#pragma unroll
+    for (int q = 0; q < SL; q++) {
+        const int r = lane + 32 * q;
+        live[q] = r < rows;
+        isu[q] = r >= n;
+        row[q] = R + (live[q] ? r : 0) * ld;
+    }
+    __syncwarp();
+    while (e < nrec) {
+        const double4 hd = fetch();
+        const int kind = __double2hiint(hd.x), col = __double2loint(hd.x) - 1, count = __double2loint(hd.y);
+        if (kind == kRecSweep) {
+            double x[SL];
+#pragma unroll
+            for (int q = 0; q < SL; q++) x[q] = row[q][col];
+            for (int j = 0; j < count; j++) {
+                const double4 cs = fetch();
+#pragma unroll
+                for (int q = 0; q < SL; q++) {
+                    const double c = isu[q] ? cs.z : cs.x, s = isu[q] ? cs.w : cs.y;
+                    const double z = row[q][col + j + 1];
+                    const double xn = (x[q] * c) + (z * s);
+                    if (live[q]) row[q][col + j] = xn;
+                    x[q] = -(x[q] * s) + (z * c);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < SL; q++)
+                if (live[q]) row[q][col + count] = x[q];
+        } else if (kind == kRecCancel) {  // columns l - 1 and i of U
+            for (int j = 0; j < count; j++) {
+                const double4 cs = fetch();
+#pragma unroll
+                for (int q = 0; q < SL; q++)
+                    if (live[q] && isu[q]) {
+                        const double y = row[q][col - 1], z = row[q][col + j];
+                        row[q][col - 1] = (y * cs.z) + (z * cs.w);
+                        row[q][col + j] = -(y * cs.w) + (z * cs.z);
+                    }
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < SL; q++)
+                if (live[q] && !isu[q]) row[q][col] = -row[q][col];
+        }
+    }
+    __syncwarp();
+    if (st.x > 0) {  // more sweeps to come
+        for (int e2 = lane; e2 < n * n; e2 += 32) Vg[e2] = R[(e2 % n) * ld + e2 / n];
+        for (int e2 = lane; e2 < kUrows * n; e2 += 32) Ug[e2] = R[(n + e2 / n) * ld + e2 % n];
+        return;
+    }
+    for (int j = lane; j < n; j += 32) W[j + 1] = B.W[(size_t)(j + 1) * B.batch + it];
+    __syncwarp();
+    const bool same = same_matrix(a, i, t);
+    const bool deriv = B.pass == 0, filt = B.pass == 1 || same;
+    if (lane == 0) {
+        const double cond = svd_cond<n>(W);
+        if (deriv && a.cond_d) a.cond_d[i] = cond;
+        if (filt && a.cond_f) a.cond_f[i] = cond;
+    }
+    // b <- V diag(1/w) U^T b; the entries of U^T b are sums over the nonzero entries of b
+    auto solve = [&](double *b, int r0, int nr, const double *coef) {
         __syncwarp();
-        const double xi = a.px[i], yi = a.py[i];
-        for (int k = lane; k < cnt; k += 32) {
-            int p = a.lpt[sell_off(a.slice_ptr, i, k)];
-            double x = -(xi - a.px[p]), y = -(yi - a.py[p]);
-            double rad = sqrt(x * x + y * y) / hh;
-            double ff1 = wab(rad, a.h2);
-            double xx = x / hh, yy = y / hh;
-            double hx[ORDER + 1], hy[ORDER + 1];
+        for (int j = lane; j < n; j += 32) {
+            double s = 0.0;
+            if (W[j + 1] != 0.0) {
+                for (int r = 0; r < nr; r++) s = s + R[(n + r0 + r) * ld + j] * coef[r];
+                s = s / W[j + 1];
+            }
+            tmp[j] = s;
+        }
+        __syncwarp();
+        for (int j = lane; j < n; j += 32) {
+            double s = 0.0;
+            for (int jj = 0; jj < n; jj++) s = s + R[j * ld + jj] * tmp[jj];
+            b[j] = s;
+        }
+        __syncwarp();
+    };
+    const double one = 1.0;
+    if (deriv) {
+        solve(bx, 0, 1, &one);
+        solve(by, 1, 1, &one);
+        solve(bxx, 2, 1, &one);
+        solve(byy, 3, 1, &one);
+        for (int m = lane; m < n; m += 32) bxx[m] = bxx[m] + byy[m];  // bvecxx + bvecyy
+    }
+    if (filt) {
+        const int fo = filter_order(a.forder, t);
+        double coef[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        int nr = 0;
+        while (nr < 6 && hyp_entry(fo, nr, &coef[nr]) >= 0) nr++;
+        solve(bh, 4, nr, coef);
+    }
+    __syncwarp();
+    const double hh = deriv ? a.hs[i] : a.h[i];
+    const double xi = a.px[i], yi = a.py[i];
+    const int cnt = a.cnt[i];
+    for (int k = lane; k < cnt; k += 32) {
+        const long long o = sell_off(a.slice_ptr, i, k);
+        const int p = a.lpt[o];
+        const double x = -(xi - a.px[p]), y = -(yi - a.py[p]);
+        const double rad = sqrt(x * x + y * y) / hh;
+        const double ff1 = wab(rad, a.h2);
+        const double xx = x / hh, yy = y / hh;
+        double hx[ORDER + 1], hy[ORDER + 1];
 #pragma unroll
-            for (int d = 0; d <= ORDER; d++) { hx[d] = hermite(d, xx); hy[d] = hermite(d, yy); }
-            double sx = 0.0, sy = 0.0, sl = 0.0;
+        for (int d = 0; d <= ORDER; d++) { hx[d] = hermite(d, xx); hy[d] = hermite(d, yy); }
+        double sx = 0.0, sy = 0.0, sl = 0.0, sh = 0.0;
 #pragma unroll
-            for (int m = 0; m < n; m++) {
-                constexpr int dummy = 0;
-                (void)dummy;
-                const int pm = p_of(m), qm = q_of(m);
-                double g = (qm == 0) ? hx[pm] : (pm == 0) ? hy[qm] : hx[pm] * hy[qm];
-                g = g * ff1;
+        for (int m = 0; m < n; m++) {
+            const int pm = p_of(m), qm = q_of(m);
+            double g = (qm == 0) ? hx[pm] : (pm == 0) ? hy[qm] : hx[pm] * hy[qm];
+            g = g * ff1;
+            if (deriv) {
                 sx = sx + bx[m] * g;
                 sy = sy + by[m] * g;
                 sl = sl + bxx[m] * g;
             }
-            long long o = sell_off(a.slice_ptr, i, k);
+            if (filt) sh = sh + bh[m] * g;
+        }
+        if (deriv) {
             a.wx[o] = sx / hh;
             a.wy[o] = sy / hh;
             a.wl[o] = (sl / hh) / hh;
         }
-        // ---- filter weights, calc_filter_weights (labf.F90:258-388) ----
-        const double hf = a.h[i];
-        const bool same = (hf == hh) && (cnt == cs) && (a.forder == a.morder) && (t != -2);
-        if (!same) {
-            assemble<ORDER>(a, i, cnt, hf, U, ld, X, G, lane);
-            if (a.forder >= 7 && (t == 998 || t < 0)) drop_order<n>(U, ld, 27, lane);
-            if (a.forder >= 5 && t == -1) drop_order<n>(U, ld, 14, lane);
-            if (svd_factor_warp<n>(U, V, W, rv1, ld, lane, a.maxits > 0 ? a.maxits : 30)) {
-                if (lane == 0) atomicExch(a.err, i + 1);
-                continue;
-            }
-            if (lane == 0) cond_d = svd_cond<n>(W);
-        }
-        if (lane == 0 && a.cond_f) a.cond_f[i] = cond_d;
-        int hord = a.forder;
-        if (a.forder >= 7 && (t == 998 || t < 0)) hord = 6;
-        if (a.forder >= 5 && t == -1) hord = 4;
-        hyp_rhs(hord, bh, n, lane);
-        svd_apply_warp<n>(U, V, W, tmp, bh, ld, lane);
-        for (int k = lane; k < cnt; k += 32) {
-            int p = a.lpt[sell_off(a.slice_ptr, i, k)];
-            double x = -(xi - a.px[p]), y = -(yi - a.py[p]);
-            double rad = sqrt(x * x + y * y) / hf;
-            double ff1 = wab(rad, a.h2);
-            double xx = x / hf, yy = y / hf;
-            double hx[ORDER + 1], hy[ORDER + 1];
-#pragma unroll
-            for (int d = 0; d <= ORDER; d++) { hx[d] = hermite(d, xx); hy[d] = hermite(d, yy); }
-            double sh = 0.0;
-#pragma unroll
-            for (int m = 0; m < n; m++) {
-                const int pm = p_of(m), qm = q_of(m);
-                double g = (qm == 0) ? hx[pm] : (pm == 0) ? hy[qm] : hx[pm] * hy[qm];
-                g = g * ff1;
-                sh = sh + bh[m] * g;
-            }
-            a.wh[sell_off(a.slice_ptr, i, k)] = sh;
-        }
-        __syncwarp();
+        if (filt) a.wh[o] = sh;
     }
 }
 
@@ -1132,25 +1635,93 @@ int smem_optin(Handle *H, int *bytes) {
     return 0;
 }
 
+// Record entries an item gets.  The jittered sets take 0.36 n^2 (order 8, at most 0.41) to
+// 0.78 n^2 (order 4, at most 0.96); what does not fit takes another round.
 template <int ORDER>
-int launch_weights(Handle *H, WArgs &a) {
-    constexpr int per_warp = smem_doubles<ORDER>() * (int)sizeof(double);
-    int optin = 0;
-    if (int rc = smem_optin(H, &optin)) return rc;
-    int wpb = optin / per_warp;
-    if (wpb > 16) wpb = 16;
-    if (wpb < 1) wpb = 1;
-    size_t smem = (size_t)wpb * per_warp;
-    SUNSET_CUDA(H, cudaFuncSetAttribute(k_labf_weights<ORDER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int nsm = 0;
-    SUNSET_CUDA(H, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, H->device));
-    int nb = (a.npfb + wpb - 1) / wpb;
-    int cap = nsm * 8;
-    if (nb > cap) nb = cap;
-    k_labf_weights<ORDER><<<nb, wpb * 32, smem, H->stream>>>(a);
-    SUNSET_CUDA(H, cudaGetLastError());
+constexpr int rec_capacity() { return nsz(ORDER) * nsz(ORDER) / 2 + 5 * nsz(ORDER) + 8; }
+// Items a batch takes: enough for k_bidiag_qr's one thread an item to hide its latency (7 warps a
+// SM), and 1.9 GB of workspace at order 8.
+constexpr int kWeightBatch = 32768;
+
+template <int ORDER>
+int weights_batches(Handle *H, const WArgs &a, SvdBatch B, const int *items, int n_items, int pass) {
+    constexpr int n = nsz(ORDER);
+    cudaStream_t st = H->stream;
+    const int maxits = a.maxits > 0 ? a.maxits : 30;
+    constexpr size_t smem1 = bidiag_doubles<ORDER>() * sizeof(double);
+    constexpr size_t smem2 = 2 * (size_t)(n + 1) * kQrThreads * sizeof(double);
+    constexpr size_t smem3 = (size_t)kApplyWarps * apply_doubles<ORDER>() * sizeof(double);
+    SUNSET_CUDA(H, cudaFuncSetAttribute(k_moment_bidiag<ORDER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1));
+    SUNSET_CUDA(H, cudaFuncSetAttribute(k_bidiag_qr<ORDER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));
+    SUNSET_CUDA(H, cudaFuncSetAttribute(k_weights_apply<ORDER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3));
+    B.pass = pass;
+    for (int b = 0; b < n_items; b += B.batch) {
+        B.item = items + b;
+        B.n_items = n_items - b < B.batch ? n_items - b : B.batch;
+        k_moment_bidiag<ORDER><<<B.n_items, bidiag_threads(ORDER), smem1, st>>>(a, B);
+        int left = 1;
+        // every round takes each item that is left at least one sweep further
+        while (left > 0) {
+            SUNSET_CUDA(H, cudaMemsetAsync(B.left, 0, sizeof(int), st));
+            k_bidiag_qr<ORDER><<<(B.n_items + kQrThreads - 1) / kQrThreads, kQrThreads, smem2, st>>>(B, maxits);
+            k_weights_apply<ORDER><<<(B.n_items + kApplyWarps - 1) / kApplyWarps, kApplyWarps * 32, smem3, st>>>(a, B);
+            SUNSET_CUDA(H, cudaGetLastError());
+            SUNSET_CUDA(H, cudaMemcpyAsync(&left, B.left, sizeof(int), cudaMemcpyDeviceToHost, st));
+            SUNSET_CUDA(H, cudaStreamSynchronize(st));
+        }
+    }
     return 0;
 }
+
+template <int ORDER>
+int launch_weights(Handle *H, WArgs &a) {
+    constexpr int n = nsz(ORDER);
+    cudaStream_t st = H->stream;
+    SvdBatch B{};
+    B.cap = rec_capacity<ORDER>();
+    int *items = nullptr, *count = nullptr;
+    char *ws = nullptr;
+    if (dalloc(H, &items, 2 * (size_t)a.npfb) || dalloc(H, &count, 4)) return SUNSET_ERR_NOMEM;
+    SUNSET_CUDA(H, cudaMemsetAsync(count, 0, 4 * sizeof(int), st));
+    k_weight_items<<<(a.npfb + 255) / 256, 256, 0, st>>>(a, items, items + a.npfb, count);
+    int hc[2] = {0, 0};
+    SUNSET_CUDA(H, cudaMemcpyAsync(hc, count, sizeof(hc), cudaMemcpyDeviceToHost, st));
+    SUNSET_CUDA(H, cudaStreamSynchronize(st));
+    // the workspace, in halves of the batch where memory is short
+    B.batch = hc[0] < kWeightBatch ? (hc[0] + 31) / 32 * 32 : kWeightBatch;
+    for (; B.batch > 0; B.batch = B.batch / 64 * 32) {
+        const size_t per = sizeof(double) * ((size_t)4 * B.cap + (kUrows + n) * n + 2 * (n + 1) + 1) + sizeof(int2) + sizeof(int);
+        void *q = nullptr;
+        if (cudaMalloc(&q, per * B.batch) == cudaSuccess) {
+            ws = static_cast<char *>(q);
+            break;
+        }
+        cudaGetLastError();
+    }
+    if (hc[0] > 0 && !ws) return set_err(H, SUNSET_ERR_NOMEM, "no memory for the weight solves");
+    int rc = 0;
+    if (ws) {
+        char *p = ws;
+        auto take = [&](size_t bytes) { char *q = p; p += bytes; return q; };
+        const size_t nb = B.batch;
+        B.rec = reinterpret_cast<double4 *>(take(nb * B.cap * sizeof(double4)));
+        B.V = reinterpret_cast<double *>(take(nb * n * n * sizeof(double)));
+        B.U = reinterpret_cast<double *>(take(nb * kUrows * n * sizeof(double)));
+        B.W = reinterpret_cast<double *>(take(nb * (n + 1) * sizeof(double)));
+        B.rv1 = reinterpret_cast<double *>(take(nb * (n + 1) * sizeof(double)));
+        B.anorm = reinterpret_cast<double *>(take(nb * sizeof(double)));
+        B.state = reinterpret_cast<int2 *>(take(nb * sizeof(int2)));
+        B.nrec = reinterpret_cast<int *>(take(nb * sizeof(int)));
+        B.left = count + 2;
+        rc = weights_batches<ORDER>(H, a, B, items, hc[0], 0);
+        if (!rc && hc[1] > 0) rc = weights_batches<ORDER>(H, a, B, items + a.npfb, hc[1], 1);
+        cudaFree(ws);
+    }
+    dfree(H, items);
+    dfree(H, count);
+    return rc;
+}
+
 
 }  // namespace
 
