@@ -341,6 +341,11 @@ int make_stream_links(Handle *H);
 void deal_slice_by_bank(int group, const uint16_t *pos, std::vector<int> *small, std::vector<int> *large,
                         const int *c_s, const int *c, int width, int *chosen);
 
+// The same order computed on the device, over sliced ELL lists: src[o] is the SELL entry whose link
+// goes to entry o (-1: padding).  width: the widest slice.
+int deal_links(Handle *H, int group, int n, int nslices, const long long *slice_ptr, const int *slice_w, const int *cnt,
+               const int *cnt_small, const uint16_t *pos, int width, int *src);
+
 int state_alloc(Handle *H);
 int state_set_device(Handle *H, const double *ro, const double *u, const double *v, const double *cxx,
                      const double *cxy, const double *cyy, const double *czz);  // internal order, device

@@ -527,10 +527,9 @@ int find_neighbours_device(Handle *H) {
 // slices (kTile nodes); its halo is the sorted set of parents its links reach.  The
 // kernels load the halo's fields once into shared memory (consecutive halo entries are
 // mostly consecutive nodes in Morton order, so these loads coalesce) and every link then
-// reads shared memory through a 16-bit position.  Built on the host once per node set.
+// reads shared memory through a 16-bit position.  Built once per node set.
 // ---------------------------------------------------------------------------------------
 #include <algorithm>
-#include <thread>
 
 namespace sunset {
 
@@ -575,63 +574,165 @@ int upload_boundary(Handle *H, const std::vector<double> &nx, const std::vector<
     return 0;
 }
 
+namespace {
+
+// The halo of one tile a block: the parents its links reach go into a hash set in shared memory
+// (tsize slots, open addressing), which is compacted and sorted.  A tile reaches a few times
+// its own nodes (700 of 256 at order 8) over ten thousand links, so nearly every link finds
+// its node already there.  count[t] is the halo's size, or -1 where the set overflowed half its
+// slots; list[t * tsize / 2 ...] the sorted nodes.
+constexpr int kHaloThreads = 256;
+__global__ void __launch_bounds__(kHaloThreads) k_tile_halos(int n, int nslices, const long long *slice_ptr, const int *cnt,
+                                                             const int *lidx, int tsize, int *list, int *count) {
+    extern __shared__ int hsm[];
+    int *table = hsm, *vals = hsm + tsize;
+    __shared__ int num;
+    const int tile = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int half = tsize / 2;
+    for (int e = tid; e < tsize; e += kHaloThreads) table[e] = -1;
+    if (tid == 0) num = 0;
+    __syncthreads();
+    const int shift = 32 - (31 - __clz(tsize));
+    for (int sl = tile * kTileSlices + warp; sl < min(nslices, (tile + 1) * kTileSlices); sl += kHaloThreads / 32) {
+        const int i = sl * kSlice + lane;
+        const int c = i < n ? cnt[i] : 0;
+        const long long base = slice_ptr[sl];
+        for (int k = 0; k < c; k++) {
+            const int p = lidx[sell_at(base, k, lane)] & kLinkMask;
+            unsigned slot = ((unsigned)p * 2654435761u) >> shift;
+            // at most half the slots fill before the tile gives up, so a free one is always near
+            for (int probe = 0; probe < tsize; probe++) {
+                int v = ((volatile int *)table)[slot];
+                if (v == p) break;
+                if (v < 0) {
+                    if (((volatile int *)&num)[0] > half) break;
+                    v = atomicCAS(&table[slot], -1, p);
+                    if (v == -1) atomicAdd(&num, 1);
+                    if (v == -1 || v == p) break;
+                }
+                slot = (slot + 1) & (tsize - 1);
+            }
+        }
+    }
+    __syncthreads();
+    const int total = num;
+    if (total > half) {
+        if (tid == 0) count[tile] = -1;
+        return;
+    }
+    __syncthreads();
+    if (tid == 0) num = 0;
+    __syncthreads();
+    for (int e = tid; e < tsize; e += kHaloThreads) {
+        const int v = table[e];
+        if (v >= 0) vals[atomicAdd(&num, 1)] = v;
+    }
+    int np2 = 1;
+    while (np2 < total) np2 <<= 1;
+    __syncthreads();
+    for (int e = total + tid; e < np2; e += kHaloThreads) vals[e] = 0x7fffffff;
+    __syncthreads();
+    for (int k = 2; k <= np2; k <<= 1)  // bitonic sort; np2 <= half, a power of two
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            for (int e = tid; e < np2; e += kHaloThreads) {
+                const int x = e ^ j;
+                if (x > e) {
+                    const int a = vals[e], b = vals[x];
+                    if ((a > b) == ((e & k) == 0)) { vals[e] = b; vals[x] = a; }
+                }
+            }
+            __syncthreads();
+        }
+    for (int e = tid; e < total; e += kHaloThreads) list[(size_t)tile * half + e] = vals[e];
+    if (tid == 0) count[tile] = total;
+}
+
+// The tiles' halos into one list, and each link's position in its tile's halo | reflection code
+// << 14 (0 in the padding), by binary search in shared memory.
+__global__ void __launch_bounds__(kHaloThreads) k_halo_links(int n, int nslices, const long long *slice_ptr, const int *slice_w,
+                                                             const int *cnt, const int *lidx, const int *list, int half,
+                                                             const int *halo_ptr, int *halo, uint16_t *lloc) {
+    extern __shared__ int hsm[];
+    const int tile = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int h0 = halo_ptr[tile], hn = halo_ptr[tile + 1] - h0;
+    for (int e = tid; e < hn; e += kHaloThreads) {
+        const int v = list[(size_t)tile * half + e];
+        hsm[e] = v;
+        halo[h0 + e] = v;
+    }
+    __syncthreads();
+    for (int sl = tile * kTileSlices + warp; sl < min(nslices, (tile + 1) * kTileSlices); sl += kHaloThreads / 32) {
+        const int i = sl * kSlice + lane;
+        const int c = i < n ? cnt[i] : 0;
+        const long long base = slice_ptr[sl];
+        const int w = slice_w[sl];
+        for (int k = 0; k < w; k += 2) {  // a pair of links is one 8-byte load and one 4-byte store
+            const long long o = sell_at(base, k, lane);
+            const int2 lk = *reinterpret_cast<const int2 *>(lidx + o);
+            unsigned out = 0;
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                if (k + q >= c) continue;
+                const int v = q ? lk.y : lk.x, p = v & kLinkMask;
+                int lo = 0, hi = hn;
+                while (hi - lo > 1) {
+                    const int mid = (lo + hi) >> 1;
+                    if (hsm[mid] <= p) lo = mid;
+                    else hi = mid;
+                }
+                out |= ((unsigned)lo | (((unsigned)v >> 30) << 14)) << (16 * q);
+            }
+            *reinterpret_cast<unsigned *>(lloc + o) = out;
+        }
+    }
+}
+
+}  // namespace
+
 int build_halos(Handle *H) {
     const int n = H->npfb, nsl = H->nslices;
     const long long L = H->nlinks_sell;
-    std::vector<int> lidx(L), cnt(n), sw(nsl);
-    std::vector<long long> sptr(nsl + 1);
-    SUNSET_CUDA(H, cudaMemcpy(lidx.data(), H->lidx, L * sizeof(int), cudaMemcpyDeviceToHost));
-    SUNSET_CUDA(H, cudaMemcpy(cnt.data(), H->cnt, n * sizeof(int), cudaMemcpyDeviceToHost));
-    SUNSET_CUDA(H, cudaMemcpy(sw.data(), H->slice_w, nsl * sizeof(int), cudaMemcpyDeviceToHost));
-    SUNSET_CUDA(H, cudaMemcpy(sptr.data(), H->slice_ptr, (nsl + 1) * sizeof(long long), cudaMemcpyDeviceToHost));
+    cudaStream_t st = H->stream;
     const int nt = (nsl + kTileSlices - 1) / kTileSlices;
-    std::vector<std::vector<int>> halos(nt);
-    std::vector<uint16_t> loc(L, 0);
-    unsigned nthr = std::max(1u, std::min(32u, std::thread::hardware_concurrency()));
-    std::vector<std::thread> pool;
-    for (unsigned w = 0; w < nthr; w++) {
-        pool.emplace_back([&, w]() {
-            for (int t = (int)w; t < nt; t += (int)nthr) {
-                std::vector<int> &hv = halos[t];
-                for (int sl = t * kTileSlices; sl < std::min(nsl, (t + 1) * kTileSlices); sl++)
-                    for (int lane = 0; lane < kSlice; lane++) {
-                        int i = sl * kSlice + lane;
-                        if (i >= n) break;
-                        for (int k = 0; k < cnt[i]; k++) hv.push_back(lidx[sell_at(sptr[sl], k, lane)] & kLinkMask);
-                    }
-                std::sort(hv.begin(), hv.end());
-                hv.erase(std::unique(hv.begin(), hv.end()), hv.end());
-                for (int sl = t * kTileSlices; sl < std::min(nsl, (t + 1) * kTileSlices); sl++)
-                    for (int lane = 0; lane < kSlice; lane++) {
-                        int i = sl * kSlice + lane;
-                        int c = i < n ? cnt[i] : 0;
-                        for (int k = 0; k < sw[sl]; k++) {
-                            long long o = sell_at(sptr[sl], k, lane);
-                            if (k >= c) { loc[o] = 0; continue; }
-                            int p = lidx[o] & kLinkMask, code = (unsigned)lidx[o] >> 30;
-                            int pos = (int)(std::lower_bound(hv.begin(), hv.end(), p) - hv.begin());
-                            loc[o] = (uint16_t)(pos | (code << 14));
-                        }
-                    }
-            }
-        });
-    }
-    for (auto &th : pool) th.join();
+    // the hash set: 4096 slots hold the halos of the orders' own stencils (2048 nodes a tile);
+    // where one is larger, 32768, the most a block's shared memory and the 14-bit index take
+    int *list = nullptr, *count = nullptr, tsize = 4096, hmax = 0;
     std::vector<int> hptr(nt + 1);
-    hptr[0] = 0;
-    int hmax = 0;
-    for (int t = 0; t < nt; t++) {
-        hptr[t + 1] = hptr[t] + (int)halos[t].size();
-        hmax = std::max(hmax, (int)halos[t].size());
+    if (dalloc(H, &count, nt)) return SUNSET_ERR_NOMEM;
+    for (;; tsize = 2 * (kLocMask + 1)) {
+        const int smem = (tsize + tsize / 2) * (int)sizeof(int);
+        if (dalloc(H, &list, (size_t)nt * (tsize / 2))) return SUNSET_ERR_NOMEM;
+        SUNSET_CUDA(H, cudaFuncSetAttribute(k_tile_halos, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        k_tile_halos<<<nt, kHaloThreads, smem, st>>>(n, nsl, H->slice_ptr, H->cnt, H->lidx, tsize, list, count);
+        SUNSET_CUDA(H, cudaGetLastError());
+        SUNSET_CUDA(H, cudaMemcpyAsync(hptr.data() + 1, count, nt * sizeof(int), cudaMemcpyDeviceToHost, st));
+        SUNSET_CUDA(H, cudaStreamSynchronize(st));
+        hptr[0] = 0;
+        hmax = 0;
+        bool over = false;
+        for (int t = 0; t < nt; t++) {
+            over = over || hptr[t + 1] < 0;
+            hmax = std::max(hmax, hptr[t + 1]);
+            hptr[t + 1] += hptr[t];
+        }
+        if (!over) break;
+        dfree(H, list);
+        if (tsize > kLocMask + 1) {
+            dfree(H, count);
+            return set_err(H, SUNSET_ERR_SCOPE, "a tile halo of more than %d nodes exceeds the 14-bit local index", kLocMask + 1);
+        }
     }
-    if (hmax > kLocMask + 1) return set_err(H, SUNSET_ERR_SCOPE, "tile halo of %d nodes exceeds the 14-bit local index", hmax);
-    std::vector<int> hall(hptr[nt]);
-    for (int t = 0; t < nt; t++) std::copy(halos[t].begin(), halos[t].end(), hall.begin() + hptr[t]);
-    if (dalloc(H, &H->halo_ptr, nt + 1) || dalloc(H, &H->halo, hall.size()) || dalloc(H, &H->lloc, L))
+    if (dalloc(H, &H->halo_ptr, nt + 1) || dalloc(H, &H->halo, (size_t)hptr[nt]) || dalloc(H, &H->lloc, L))
         return SUNSET_ERR_NOMEM;
-    SUNSET_CUDA(H, cudaMemcpyAsync(H->halo_ptr, hptr.data(), hptr.size() * sizeof(int), cudaMemcpyHostToDevice, H->stream));
-    SUNSET_CUDA(H, cudaMemcpyAsync(H->halo, hall.data(), hall.size() * sizeof(int), cudaMemcpyHostToDevice, H->stream));
-    SUNSET_CUDA(H, cudaMemcpyAsync(H->lloc, loc.data(), L * sizeof(uint16_t), cudaMemcpyHostToDevice, H->stream));
+    SUNSET_CUDA(H, cudaMemcpyAsync(H->halo_ptr, hptr.data(), hptr.size() * sizeof(int), cudaMemcpyHostToDevice, st));
+    const int smem = hmax * (int)sizeof(int);
+    SUNSET_CUDA(H, cudaFuncSetAttribute(k_halo_links, cudaFuncAttributeMaxDynamicSharedMemorySize, (kLocMask + 1) * (int)sizeof(int)));
+    k_halo_links<<<nt, kHaloThreads, smem, st>>>(n, nsl, H->slice_ptr, H->slice_w, H->cnt, H->lidx, list, tsize / 2,
+                                                 H->halo_ptr, H->halo, H->lloc);
+    SUNSET_CUDA(H, cudaGetLastError());
+    SUNSET_CUDA(H, cudaStreamSynchronize(st));
+    dfree(H, list);
+    dfree(H, count);
     H->ntiles = nt;
     H->halo_max = hmax;
     return 0;

@@ -8,7 +8,7 @@
 // gather the tile halo from shared memory with 8-byte loads, which are served per
 // half-warp, one wavefront per bank pair (position mod 16) and distinct position.  In the
 // reference order neighbouring lanes often meet in the same bank pair at the same link slot
-// (4.9 wavefronts a load on the order-6 set against the ideal 2).  order_links_by_bank()
+// (4.9 wavefronts a load on the order-6 set against the ideal 2).  k_deal_links
 // re-deals each node's links slot by slot so that the 16 lanes of a half-warp read distinct
 // bank pairs wherever a bipartite matching allows it (2.6 on that set).  Only the rounding
 // of the sums changes (relative 1e-16 a sum).
@@ -27,7 +27,6 @@
 // nodes -- and acts as a small extra Laplacian, 1e-6 of the fields in 100 steps.)
 // The filter streams its weight rounded to FP32 with the local index (6 bytes a link).
 #include <algorithm>
-#include <thread>
 #include <vector>
 
 #include "internal.cuh"
@@ -120,51 +119,160 @@ __global__ void k_stream_weights(StreamArgs a) {
     }
 }
 
+// deal_slice_by_bank (bank_deal.cu) on the device, one warp a slice, with the same result: slot
+// by slot, the lanes of each group of G are matched to the G bank groups by augmenting paths,
+// the most constrained lane first, each lane trying its bank groups in the list order of their
+// first remaining link.  src[o]: the SELL entry (in the reference order) whose link goes to
+// entry o, or -1 for padding.
+//
+// A thread plays two parts: lane r of its group (the links it has left, the bank group it takes)
+// and bank group t (its owner).  The groups of a warp take the steps of their searches side by
+// side: in one step a lane's next bank group is the smallest first link, over the group's
+// threads, among the bank groups not tried yet.  A search tries a bank group once, so it ends
+// after at most 2 G steps.  Bound: the latency of those steps (a shared load, four shuffles),
+// hidden by the slices of the set.  1,048,576 nodes at order 8: the host's threads took
+// 0.9-2.0 s with their copies both ways.
+constexpr unsigned short kNoLink = 0xffff;
+constexpr int kDealWarps = 4;
+__host__ __device__ inline int deal_smem(int width) { return (width * 32 + 2 * 32 * 16) * (int)sizeof(unsigned short); }
+
+template <int G>
+__global__ void __launch_bounds__(kDealWarps * 32) k_deal_links(int n, int nslices, const long long *slice_ptr, const int *slice_w,
+                                                                const int *cnt, const int *cnt_small, const uint16_t *pos,
+                                                                int width, int *src) {
+    extern __shared__ unsigned short dsm[];
+    const unsigned all = 0xffffffffu, gmask = (1u << G) - 1u;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int sl = blockIdx.x * (blockDim.x >> 5) + warp;
+    if (sl >= nslices) return;
+    const int t = lane & (G - 1), g0 = lane - t;
+    unsigned short *nxt = dsm + (size_t)warp * (deal_smem(width) / sizeof(unsigned short));  // next link of the same bank group
+    unsigned short *fr = nxt + width * 32, *fr2 = fr + 32 * 16;  // first link by lane and bank group: current set, other links
+    const int i = sl * kSlice + lane;
+    const int c = i < n ? cnt[i] : 0, cs = i < n ? min(cnt_small[i], c) : 0;
+    const long long base = slice_ptr[sl];
+    const int w = slice_w[sl];
+    unsigned mask = 0, mask2 = 0;  // bank groups that the lane has links of
+    for (int b = 0; b < 16; b++) fr[lane * 16 + b] = fr2[lane * 16 + b] = kNoLink;
+    for (int k = c - 1; k >= 0; k--) {
+        const int b = pos[sell_at(base, k, lane)] & (G - 1);
+        unsigned short *f = (k < cs ? fr : fr2) + lane * 16 + b;
+        nxt[k * 32 + lane] = *f;
+        *f = (unsigned short)k;
+        if (k < cs) mask |= 1u << b;
+        else mask2 |= 1u << b;
+    }
+    for (int k = 0; k < w; k++) {
+        if (k == cs && cs < c) {  // the small links are dealt: go on with the others
+            for (int b = 0; b < 16; b++) fr[lane * 16 + b] = fr2[lane * 16 + b];
+            mask = mask2;
+        }
+        __syncwarp();
+        const bool has = k < c;
+        // rank of the lane: fewest bank groups first, then lane order
+        const int key = has ? __popc(mask) * 32 + t : 0x10000;
+        int rank = 0;
+#pragma unroll
+        for (int j = 0; j < G; j++) rank += __shfl_sync(all, key, g0 + j) < key;
+        if (!has) rank = 99;
+        const int nact = __popc((__ballot_sync(all, has) >> g0) & gmask);
+        int owner = (t == 0 && nact < G) ? G : -1;  // padding lanes read position 0
+        int choice = -1;
+        int q = 0, r = -1, depth = 0, sr = 0, sb = 0;
+        unsigned seen = 0;
+        while (__any_sync(all, q < nact)) {
+            const bool run = q < nact;
+            const int rq = __ffs((__ballot_sync(all, rank == q) >> g0) & gmask) - 1;
+            if (run && r < 0) {
+                r = rq;
+                seen = 0;
+            }
+            unsigned v = run ? fr[(g0 + r) * 16 + t] : kNoLink;
+            v = (v != kNoLink && !((seen >> t) & 1u)) ? (v << 4 | t) : 0xffffffffu;
+#pragma unroll
+            for (int o = G / 2; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(all, v, o));
+            const bool found = run && v != 0xffffffffu;
+            const int b = v & 15;
+            const int ob = __shfl_sync(all, owner, g0 + (found ? b : 0));
+            const int back = __shfl_sync(all, sr, g0 + (depth > 0 ? depth - 1 : 0));
+            const bool won = found && ob < 0;
+            if (__any_sync(all, won)) {  // each lane of the path takes the bank group it was trying
+                if (won && t == b) owner = r;
+                if (won && t == r) choice = b;
+                for (int d = depth - 1; __any_sync(all, won && d >= 0); d--) {
+                    const int pr = __shfl_sync(all, sr, g0 + (d > 0 ? d : 0)), pb = __shfl_sync(all, sb, g0 + (d > 0 ? d : 0));
+                    if (won && d >= 0) {
+                        if (t == pb) owner = pr;
+                        if (t == pr) choice = pb;
+                    }
+                }
+            }
+            if (found) seen |= 1u << b;
+            if (won || (run && !found && depth == 0)) {  // matched, or left without a match
+                q++;
+                r = -1;
+                depth = 0;
+            } else if (run && !found) {
+                depth--;
+                r = back;
+            } else if (found && ob < G) {  // the owner looks for another bank group
+                if (t == depth) {
+                    sr = r;
+                    sb = b;
+                }
+                depth++;
+                r = ob;
+            }
+        }
+        if (__any_sync(all, has && choice < 0)) {  // unmatched lanes: the least used bank group, in list order
+            int used = owner >= 0 ? 1 : 0;
+            for (q = 0; __any_sync(all, q < nact); q++) {
+                const int rq = __ffs((__ballot_sync(all, rank == q) >> g0) & gmask) - 1;
+                const int at = rq > 0 ? rq : 0;
+                const bool open = __shfl_sync(all, choice, g0 + at) < 0 && q < nact;
+                unsigned v = open ? fr[(g0 + at) * 16 + t] : kNoLink;
+                v = v != kNoLink ? ((unsigned)used << 20 | v << 4 | t) : 0xffffffffu;
+#pragma unroll
+                for (int o = G / 2; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(all, v, o));
+                if (open && t == at) choice = v & 15;
+                if (open && t == (int)(v & 15)) used++;
+            }
+        }
+        __syncwarp();
+        int from = -1;
+        if (has) {
+            const int e = fr[lane * 16 + choice];
+            const unsigned short nx = nxt[e * 32 + lane];
+            fr[lane * 16 + choice] = nx;
+            if (nx == kNoLink) mask &= ~(1u << choice);
+            from = (int)sell_at(base, e, lane);
+        }
+        src[sell_at(base, k, lane)] = from;
+    }
+}
+
+template <int G>
+int launch_deal(Handle *H, int n, int nslices, const long long *slice_ptr, const int *slice_w, const int *cnt,
+                const int *cnt_small, const uint16_t *pos, int width, int *src, cudaStream_t st) {
+    const int per = deal_smem(width), most = 200 * 1024;
+    if (per > most) return set_err(H, SUNSET_ERR_SCOPE, "neighbour lists too long for the link order");
+    const int warps = std::max(1, std::min(kDealWarps, (48 * 1024) / per));
+    SUNSET_CUDA(H, cudaFuncSetAttribute(k_deal_links<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    k_deal_links<G><<<(nslices + warps - 1) / warps, warps * 32, warps * per, st>>>(n, nslices, slice_ptr, slice_w, cnt,
+                                                                                   cnt_small, pos, width, src);
+    SUNSET_CUDA(H, cudaGetLastError());
+    return 0;
+}
+
 }  // namespace
 
-// New SELL order of the links for the time step: src[o] = the SELL entry (in the reference
-// order) whose link goes to entry o, or -1 for padding.  Small links stay in the slots
-// [0, cnt_small) and the other links in [cnt_small, cnt), so the stage kernel (small links)
-// and the filter (all links) see the same sets as in the reference order.
-static int order_links_by_bank(Handle *H, std::vector<int> &src) {
-    const int n = H->npfb, nsl = H->nslices;
-    const long long L = H->nlinks_sell;
-    std::vector<uint16_t> loc(L);
-    std::vector<int> cnt(n), cs(n), sw(nsl);
-    std::vector<long long> sptr(nsl + 1);
-    SUNSET_CUDA(H, cudaMemcpy(loc.data(), H->lloc, L * sizeof(uint16_t), cudaMemcpyDeviceToHost));
-    SUNSET_CUDA(H, cudaMemcpy(cnt.data(), H->cnt, n * sizeof(int), cudaMemcpyDeviceToHost));
-    SUNSET_CUDA(H, cudaMemcpy(cs.data(), H->cnt_small, n * sizeof(int), cudaMemcpyDeviceToHost));
-    SUNSET_CUDA(H, cudaMemcpy(sw.data(), H->slice_w, nsl * sizeof(int), cudaMemcpyDeviceToHost));
-    SUNSET_CUDA(H, cudaMemcpy(sptr.data(), H->slice_ptr, (nsl + 1) * sizeof(long long), cudaMemcpyDeviceToHost));
-    src.assign(L, -1);
-    const unsigned nthr = std::max(1u, std::min(32u, std::thread::hardware_concurrency()));
-    std::vector<std::thread> pool;
-    for (unsigned w = 0; w < nthr; w++) {
-        pool.emplace_back([&, w]() {
-            std::vector<int> small[kSlice], large[kSlice];
-            std::vector<int> chosen;
-            for (int sl = (int)w; sl < nsl; sl += (int)nthr) {
-                int c[kSlice], c_s[kSlice];
-                for (int lane = 0; lane < kSlice; lane++) {
-                    const int i = sl * kSlice + lane;
-                    c[lane] = i < n ? cnt[i] : 0;
-                    c_s[lane] = i < n ? std::min(cs[i], c[lane]) : 0;
-                    small[lane].clear();
-                    large[lane].clear();
-                    for (int k = 0; k < c[lane]; k++)
-                        (k < c_s[lane] ? small[lane] : large[lane]).push_back((int)sell_at(sptr[sl], k, lane));
-                }
-                chosen.assign((size_t)sw[sl] * kSlice, -1);
-                deal_slice_by_bank(16, loc.data(), small, large, c_s, c, sw[sl], chosen.data());
-                for (int k = 0; k < sw[sl]; k++)
-                    for (int lane = 0; lane < kSlice; lane++)
-                        if (chosen[k * kSlice + lane] >= 0) src[sell_at(sptr[sl], k, lane)] = chosen[k * kSlice + lane];
-            }
-        });
-    }
-    for (auto &th : pool) th.join();
-    return 0;
+// New SELL order of the links for the time step: small links stay in the slots [0, cnt_small)
+// and the other links in [cnt_small, cnt), so the stage kernel (small links) and the filter
+// (all links) see the same sets as in the reference order.
+int deal_links(Handle *H, int group, int n, int nslices, const long long *slice_ptr, const int *slice_w, const int *cnt,
+               const int *cnt_small, const uint16_t *pos, int width, int *src) {
+    return group == 16 ? launch_deal<16>(H, n, nslices, slice_ptr, slice_w, cnt, cnt_small, pos, width, src, H->stream)
+                       : launch_deal<8>(H, n, nslices, slice_ptr, slice_w, cnt, cnt_small, pos, width, src, H->stream);
 }
 
 // Called once the FP64 weights, their sums and the filter coefficients exist.
@@ -184,11 +292,11 @@ int make_stream_links(Handle *H) {
                 return SUNSET_ERR_NOMEM;
         }
     }
-    std::vector<int> src;
-    if (int rc = order_links_by_bank(H, src)) return rc;
     int *d_src = nullptr;
     if (dalloc(H, &d_src, L)) return SUNSET_ERR_NOMEM;
-    SUNSET_CUDA(H, cudaMemcpyAsync(d_src, src.data(), L * sizeof(int), cudaMemcpyHostToDevice, H->stream));
+    if (int rc = deal_links(H, 16, n, H->nslices, H->slice_ptr, H->slice_w, H->cnt, H->cnt_small, H->lloc,
+                            (H->nplink + 1) & ~1, d_src))
+        return rc;
     StreamArgs a{n, H->slice_ptr, H->slice_w, d_src, H->lloc, H->wx, H->wy, H->wl, H->wh, H->lloc_s,
                  H->wx_s, H->wy_s, H->wl_s, H->wh_s, H->pk, H->scx, H->scy, H->scl, H->wf};
     if (mx) k_stream_weights<true><<<(n + 255) / 256, 256, 0, H->stream>>>(a);
@@ -200,3 +308,30 @@ int make_stream_links(Handle *H) {
 }
 
 }  // namespace sunset
+
+// The device's link order on host arrays in the SELL layout, for the test that compares it with
+// deal_slice_by_bank (not part of the interface in include/sunset_gpu.h).
+extern "C" int sunset_check_deal(int group, int nslices, const long long *slice_ptr, const int *slice_w, const int *cnt,
+                                 const int *cnt_small, const uint16_t *pos, int width, int *src) {
+    using namespace sunset;
+    Handle H;
+    const int n = nslices * kSlice;
+    const size_t L = (size_t)slice_ptr[nslices];
+    long long *dp;
+    int *dw, *dc, *ds, *dsrc;
+    uint16_t *dpos;
+    int rc = SUNSET_ERR_NOMEM;
+    if (!dalloc(&H, &dp, nslices + 1) && !dalloc(&H, &dw, nslices) && !dalloc(&H, &dc, n) && !dalloc(&H, &ds, n) &&
+        !dalloc(&H, &dpos, L) && !dalloc(&H, &dsrc, L)) {
+        cudaMemcpy(dp, slice_ptr, (nslices + 1) * sizeof(long long), cudaMemcpyHostToDevice);
+        cudaMemcpy(dw, slice_w, nslices * sizeof(int), cudaMemcpyHostToDevice);
+        cudaMemcpy(dc, cnt, n * sizeof(int), cudaMemcpyHostToDevice);
+        cudaMemcpy(ds, cnt_small, n * sizeof(int), cudaMemcpyHostToDevice);
+        cudaMemcpy(dpos, pos, L * sizeof(uint16_t), cudaMemcpyHostToDevice);
+        cudaDeviceSynchronize();
+        rc = deal_links(&H, group, n, nslices, dp, dw, dc, ds, dpos, width, dsrc);
+        if (!rc && cudaMemcpy(src, dsrc, L * sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) rc = SUNSET_ERR_CUDA;
+    }
+    while (!H.allocs.empty()) dfree(&H, H.allocs.back());
+    return rc;
+}

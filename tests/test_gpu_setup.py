@@ -1,17 +1,56 @@
-"""The weight build at the sizes where it can go wrong: several batches, second rounds, order 10.
+"""The set-up kernels at the sizes where they can go wrong: the device's bank-aware link order
+against the host's, the weight build over several batches and at order 10, and the tile halos
+of a stencil too wide for the smaller hash set.
 
-The weights are compared bit for bit with the restatement (both round every operation alike, with
-its correctly rounded x^4), except the filter's, which CUDA's and glibc's cos separate in the
-last bit (1e-13, as in the parity tests).
+The link order is compared entry by entry; the weights bit for bit with the restatement (both
+round every operation alike, with its correctly rounded x^4), except the filter's, which CUDA's
+and glibc's cos separate in the last bit (1e-13, as in the parity tests); the right-hand
+sides of the wide stencil, whose sums run in another order, within 1e-10 of their terms.
 """
+import ctypes as C
+import os
+
 import numpy as np
 import pytest
 
 from sunset_viscoelastic_b200 import labfm
-from sunset_viscoelastic_b200.nodesets import jittered_lattice
+from sunset_viscoelastic_b200.nodesets import initial_state, jittered_lattice
 import oracle as O
 
 pytestmark = pytest.mark.gpu
+HOSTCHECK = os.path.join(os.path.dirname(labfm.library_path()), "libsunset_hostcheck.so")
+
+
+def sell_at(base, k, lane):
+    return base + ((k >> 1) << 6) + (lane << 1) + (k & 1)
+
+
+# (links a lane at most, slices, lanes without links, share of small links)
+@pytest.mark.parametrize("group", [8, 16])
+@pytest.mark.parametrize("most,slices,empty,small", [(1, 3, 0, 1.0), (2, 5, 31, 0.5), (37, 7, 5, 0.6), (92, 6, 0, 1.0),
+                                                     (92, 5, 3, 0.0), (333, 2, 1, 0.8)])
+def test_link_order_equals_the_hosts(group, most, slices, empty, small):
+    rng = np.random.default_rng(most + group)
+    cnt = rng.integers(max(1, most // 2), most + 1, (slices, 32)).astype(np.int32)
+    cnt[-1, 32 - empty:] = 0
+    cs = np.floor(cnt * np.minimum(1.0, small + 0.1 * rng.random(cnt.shape) * (small not in (0.0, 1.0)))).astype(np.int32)
+    w = ((cnt.max(1) + 1) & ~1).astype(np.int32)
+    ptr = np.concatenate([[0], np.cumsum(32 * w.astype(np.int64))])
+    pos = rng.integers(0, 900, int(ptr[-1])).astype(np.uint16)
+    pos[rng.random(pos.size) < 0.2] |= np.uint16(1 << 14)  # reflection codes ride in the top bits
+    lib, host = labfm.load_library(), C.CDLL(HOSTCHECK)
+    p = lambda a: a.ctypes.data_as(C.c_void_p)
+    got = np.full(int(ptr[-1]), -7, np.int32)
+    assert lib.sunset_check_deal(group, slices, p(ptr), p(w), p(cnt), p(cs), p(pos), int(w.max()), p(got)) == 0
+    for s in range(slices):
+        lists = [[[sell_at(int(ptr[s]), k, r) for k in range(*rng_)] for r, rng_ in enumerate(rows)]
+                 for rows in ([(0, int(cs[s, r])) for r in range(32)], [(int(cs[s, r]), int(cnt[s, r])) for r in range(32)])]
+        flat = [np.array([e for row in rows for e in row] or [0], np.int32) for rows in lists]
+        off = [np.concatenate([[0], np.cumsum([len(row) for row in rows])]).astype(np.int32) for rows in lists]
+        want = np.full(int(w[s]) * 32, -7, np.int32)
+        host.sunset_hostcheck_deal(group, p(pos), p(flat[0]), p(off[0]), p(flat[1]), p(off[1]), int(w[s]), p(want))
+        mine = np.array([[got[sell_at(int(ptr[s]), k, r)] for r in range(32)] for k in range(int(w[s]))])
+        assert np.array_equal(mine, want.reshape(-1, 32))
 
 
 def pair(ns, order, h_over_s, **kw):
@@ -32,3 +71,16 @@ def test_weights_equal_the_restatements(order, nside, radius):
     for k in ("w_grad", "w_lap", "w_grad_sum", "w_lap_sum"):
         assert np.array_equal(a[k], b[k]), k
     assert np.abs(a["w_hyp"] - b["w_hyp"]).max() <= 1e-13 * np.abs(b["w_hyp"]).max()
+
+
+def test_wide_stencil_halos():
+    ns = jittered_lattice(64)
+    ref, gpu = pair(ns, 4, 15.5 / 2)
+    st = initial_state(ns)
+    st["cxx"] = 1.0 + 0.2 * np.sin(2 * np.pi * ns.x)
+    for g in (ref, gpu):
+        g.set_state(**st)
+    a, b = gpu.rhs(), ref.rhs()
+    # the largest term: the viscous force, (1 / s^2) |u|, and the pressure gradient, c^2 |grad rho|
+    for k in ("ro", "rou", "rov", "xx", "xy", "yy"):
+        assert np.abs(a[k] - b[k]).max() <= 1e-10 * max(1.0, np.abs(b[k]).max()), k
