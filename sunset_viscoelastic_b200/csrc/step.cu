@@ -1864,6 +1864,11 @@ int state_alloc(Handle *H) {
         }
         if (H->cfg.fenep && (H->cfg.form == SUNSET_FORM_DI || H->cfg.form == SUNSET_FORM_LC) && dalloc(H, &F.f, n))
             return SUNSET_ERR_NOMEM;
+        // the Newtonian form never writes these, and they are exported
+        for (int k = 0; k < 4; k++) {
+            SUNSET_CUDA(H, cudaMemsetAsync(F.q[k], 0, n * sizeof(double), H->stream));
+            SUNSET_CUDA(H, cudaMemsetAsync(F.c[k], 0, n * sizeof(double), H->stream));
+        }
     }
     for (int f = 0; f < 7; f++) {
         if (dalloc(H, &H->rhs[f], n)) return SUNSET_ERR_NOMEM;
