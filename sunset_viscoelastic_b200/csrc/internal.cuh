@@ -21,6 +21,7 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <map>
 #include <string>
 #include <vector>
 
@@ -292,7 +293,14 @@ struct Handle {
     double adj_graph_dt = 0.0;                 // dt and checkpoint store the two graphs were captured with
     const double *adj_graph_cp = nullptr;
 
-    std::vector<void *> allocs;
+    // device memory of the handle (abi.cu): blocks with their free ranges, and the pieces given out
+    struct Block {
+        char *base;
+        size_t size;
+        std::map<size_t, size_t> free;  // offset -> length
+    };
+    std::vector<Block> blocks;
+    std::map<void *, size_t> allocs;
 };
 
 // error helpers
@@ -305,16 +313,24 @@ int set_err(Handle *H, int code, const char *fmt, ...);
                                      cudaGetErrorString(e_), __FILE__, __LINE__);               \
     } while (0)
 
+// Device memory of the handle: 256-byte aligned pieces of its blocks, null when there is none
+// left.  A freed piece may be given out again at once, so every kernel and copy that touches one
+// runs on the handle's stream (or has been waited for).
+void *device_alloc(Handle *H, size_t bytes);
 template <typename T>
 int dalloc(Handle *H, T **p, size_t n) {
-    void *q = nullptr;
-    cudaError_t e = cudaMalloc(&q, (n ? n : 1) * sizeof(T));
-    if (e != cudaSuccess) return set_err(H, SUNSET_ERR_NOMEM, "cudaMalloc(%zu) failed: %s", n * sizeof(T), cudaGetErrorString(e));
-    H->allocs.push_back(q);
+    void *q = device_alloc(H, (n ? n : 1) * sizeof(T));
+    if (!q) return set_err(H, SUNSET_ERR_NOMEM, "no device memory for %zu bytes", n * sizeof(T));
     *p = static_cast<T *>(q);
     return 0;
 }
 void dfree(Handle *H, void *p);
+void dfree_all(Handle *H);
+// device -> host on the handle's stream, waited for
+inline cudaError_t copy_out(Handle *H, void *dst, const void *src, size_t bytes) {
+    cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, H->stream);
+    return e != cudaSuccess ? e : cudaStreamSynchronize(H->stream);
+}
 
 // stage entry points implemented in the .cu files
 int build_domain_device(Handle *H, const std::vector<double> &x, const std::vector<double> &y,

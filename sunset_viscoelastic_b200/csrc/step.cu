@@ -2065,7 +2065,7 @@ int time_stage_kernel(Handle *H, int reps, double *ms, double *bytes) {
     long long links = 0;
     {
         std::vector<int> cs(H->npfb);
-        SUNSET_CUDA(H, cudaMemcpy(cs.data(), H->cnt_small, cs.size() * sizeof(int), cudaMemcpyDeviceToHost));
+        SUNSET_CUDA(H, copy_out(H, cs.data(), H->cnt_small, cs.size() * sizeof(int)));
         for (int c : cs) links += c;
     }
     const int form = H->cfg.form;
@@ -2152,8 +2152,8 @@ size_t checkpoint_bytes(const Handle *H) {
 
 static int node_fingerprint(Handle *H, double *xs, double *ys) {
     std::vector<double> x(H->npfb), y(H->npfb);
-    SUNSET_CUDA(H, cudaMemcpy(x.data(), H->px, H->npfb * sizeof(double), cudaMemcpyDeviceToHost));
-    SUNSET_CUDA(H, cudaMemcpy(y.data(), H->py, H->npfb * sizeof(double), cudaMemcpyDeviceToHost));
+    SUNSET_CUDA(H, copy_out(H, x.data(), H->px, H->npfb * sizeof(double)));
+    SUNSET_CUDA(H, copy_out(H, y.data(), H->py, H->npfb * sizeof(double)));
     double a = 0.0, b = 0.0;
     for (int i = 0; i < H->npfb; i++) { a = a + x[i]; b = b + y[i]; }
     *xs = a;
@@ -2644,10 +2644,10 @@ static int adjoint_build_reverse(Handle *H) {
     const long long L = H->nlinks_sell;
     std::vector<int> lidx(L), cnt(n), cs(n);
     std::vector<long long> sptr(nsl + 1);
-    SUNSET_CUDA(H, cudaMemcpy(lidx.data(), H->lidx, L * sizeof(int), cudaMemcpyDeviceToHost));
-    SUNSET_CUDA(H, cudaMemcpy(cnt.data(), H->cnt, n * sizeof(int), cudaMemcpyDeviceToHost));
-    SUNSET_CUDA(H, cudaMemcpy(cs.data(), H->cnt_small, n * sizeof(int), cudaMemcpyDeviceToHost));
-    SUNSET_CUDA(H, cudaMemcpy(sptr.data(), H->slice_ptr, (nsl + 1) * sizeof(long long), cudaMemcpyDeviceToHost));
+    SUNSET_CUDA(H, copy_out(H, lidx.data(), H->lidx, L * sizeof(int)));
+    SUNSET_CUDA(H, copy_out(H, cnt.data(), H->cnt, n * sizeof(int)));
+    SUNSET_CUDA(H, copy_out(H, cs.data(), H->cnt_small, n * sizeof(int)));
+    SUNSET_CUDA(H, copy_out(H, sptr.data(), H->slice_ptr, (nsl + 1) * sizeof(long long)));
     std::vector<long long> rptr(n + 1, 0);
     for (int i = 0; i < n; i++)
         for (int k = 0; k < cnt[i]; k++) rptr[(lidx[sell_at(sptr[i >> 5], k, i & 31)] & kLinkMask) + 1]++;
@@ -2695,13 +2695,13 @@ static int adjoint_build_stream(Handle *H) {
     if (H->rv_sptr) return 0;
     const int n = H->npfb, nsl = H->nslices;
     std::vector<long long> rptr(n + 1);
-    SUNSET_CUDA(H, cudaMemcpy(rptr.data(), H->rptr, (n + 1) * sizeof(long long), cudaMemcpyDeviceToHost));
+    SUNSET_CUDA(H, copy_out(H, rptr.data(), H->rptr, (n + 1) * sizeof(long long)));
     const long long ne = rptr[n];
     std::vector<int> rslot(ne), rnode(ne);
     std::vector<unsigned char> rcode(ne);
-    SUNSET_CUDA(H, cudaMemcpy(rslot.data(), H->rslot, ne * sizeof(int), cudaMemcpyDeviceToHost));
-    SUNSET_CUDA(H, cudaMemcpy(rnode.data(), H->rnode, ne * sizeof(int), cudaMemcpyDeviceToHost));
-    SUNSET_CUDA(H, cudaMemcpy(rcode.data(), H->rcode, ne * sizeof(unsigned char), cudaMemcpyDeviceToHost));
+    SUNSET_CUDA(H, copy_out(H, rslot.data(), H->rslot, ne * sizeof(int)));
+    SUNSET_CUDA(H, copy_out(H, rnode.data(), H->rnode, ne * sizeof(int)));
+    SUNSET_CUDA(H, copy_out(H, rcode.data(), H->rcode, ne * sizeof(unsigned char)));
     std::vector<long long> sptr(nsl + 1, 0);
     std::vector<int> sw(nsl), sws(nsl);
     for (int sl = 0; sl < nsl; sl++) {

@@ -1448,7 +1448,7 @@ int layers_set(Handle *H, double Lz) {
     // build_3rd_dimension, setup_domain.F90:444-483: dz from the mean spacing (s^3 over s^2,
     // summed in the reference's node order), then nz layers over L_domain_z
     std::vector<double> sp(H->npfb);
-    SUNSET_CUDA(H, cudaMemcpy(sp.data(), H->sp, H->npfb * sizeof(double), cudaMemcpyDeviceToHost));
+    SUNSET_CUDA(H, copy_out(H, sp.data(), H->sp, H->npfb * sizeof(double)));
     std::vector<double> sref(H->npfb);
     for (int i = 0; i < H->npfb; i++) sref[H->h_perm[i]] = sp[i];
     double dzl = 0.0, sv = 0.0;
@@ -1767,8 +1767,8 @@ static int checkpoint3_header(Handle *H, Checkpoint3Header &hd) {
     hd.nb = H->nb;
     hd.dz = H->dz;
     std::vector<double> x(H->npfb), y(H->npfb);
-    SUNSET_CUDA(H, cudaMemcpy(x.data(), H->px, H->npfb * sizeof(double), cudaMemcpyDeviceToHost));
-    SUNSET_CUDA(H, cudaMemcpy(y.data(), H->py, H->npfb * sizeof(double), cudaMemcpyDeviceToHost));
+    SUNSET_CUDA(H, copy_out(H, x.data(), H->px, H->npfb * sizeof(double)));
+    SUNSET_CUDA(H, copy_out(H, y.data(), H->py, H->npfb * sizeof(double)));
     for (int i = 0; i < H->npfb; i++) { hd.xsum = hd.xsum + x[i]; hd.ysum = hd.ysum + y[i]; }
     return 0;
 }
@@ -1866,7 +1866,7 @@ int ke_mass3(Handle *H, double *ke, double *mass) {
 int time3_derivs(Handle *H, int reps, double *ms, double *bytes) {
     if (reps < 1) reps = 1;
     DevScalars s;
-    SUNSET_CUDA(H, cudaMemcpy(&s, H->dsc, sizeof(s), cudaMemcpyDeviceToHost));
+    SUNSET_CUDA(H, copy_out(H, &s, H->dsc, sizeof(s)));
     std::vector<cudaEvent_t> ev(8 * (size_t)reps);
     for (auto &e : ev) SUNSET_CUDA(H, cudaEventCreate(&e));
     int rc = step3_run(H, s.dt, reps, 0, ev.data());
@@ -1895,7 +1895,7 @@ int time3_derivs(Handle *H, int reps, double *ms, double *bytes) {
     long long links = 0;
     {
         std::vector<int> cs(H->npfb);
-        SUNSET_CUDA(H, cudaMemcpy(cs.data(), H->cnt_small, cs.size() * sizeof(int), cudaMemcpyDeviceToHost));
+        SUNSET_CUDA(H, copy_out(H, cs.data(), H->cnt_small, cs.size() * sizeof(int)));
         for (int c : cs) links += c;
     }
     const double fen = (form == SUNSET_FORM_DI && H->cfg.fenep) ? 8.0 : 0.0;

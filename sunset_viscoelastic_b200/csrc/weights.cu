@@ -1691,12 +1691,8 @@ int launch_weights(Handle *H, WArgs &a) {
     B.batch = hc[0] < kWeightBatch ? (hc[0] + 31) / 32 * 32 : kWeightBatch;
     for (; B.batch > 0; B.batch = B.batch / 64 * 32) {
         const size_t per = sizeof(double) * ((size_t)4 * B.cap + (kUrows + n) * n + 2 * (n + 1) + 1) + sizeof(int2) + sizeof(int);
-        void *q = nullptr;
-        if (cudaMalloc(&q, per * B.batch) == cudaSuccess) {
-            ws = static_cast<char *>(q);
-            break;
-        }
-        cudaGetLastError();
+        ws = static_cast<char *>(device_alloc(H, per * B.batch));
+        if (ws) break;
     }
     if (hc[0] > 0 && !ws) return set_err(H, SUNSET_ERR_NOMEM, "no memory for the weight solves");
     int rc = 0;
@@ -1715,7 +1711,7 @@ int launch_weights(Handle *H, WArgs &a) {
         B.left = count + 2;
         rc = weights_batches<ORDER>(H, a, B, items, hc[0], 0);
         if (!rc && hc[1] > 0) rc = weights_batches<ORDER>(H, a, B, items + a.npfb, hc[1], 1);
-        cudaFree(ws);
+        dfree(H, ws);
     }
     dfree(H, items);
     dfree(H, count);
