@@ -202,9 +202,9 @@ struct Handle {
     int *lpt = nullptr;                        // SELL: point id (ghost-aware), for setup/export
     int *lidx = nullptr;                       // SELL: parent | vrel code << 30
     bool has_mirrors = false;
-    // tiles of kTileSlices slices: the sorted set of nodes their links reach (the halo) and,
+    // tiles of tslices slices (kTileSlices, or fewer on small sets): the sorted set of nodes their links reach (the halo) and,
     // per link, the position of its parent in that set | reflection code << 14
-    int ntiles = 0, halo_max = 0;
+    int ntiles = 0, halo_max = 0, tslices = kTileSlices;
     int *halo_ptr = nullptr, *halo = nullptr;
     uint16_t *lloc = nullptr;
 
@@ -277,7 +277,7 @@ struct Handle {
     int *rv_sw = nullptr, *rv_sws = nullptr;   // slice widths: all links, small links
     uint16_t *rv_loc_s = nullptr, *rv_loc_f = nullptr;
     int *rv_hptr = nullptr, *rv_halo = nullptr;
-    int rv_hmax = 0;
+    int rv_hmax = 0, rv_ntiles = 0;  // its tiles have kTileSlices slices
     double *rv_wx = nullptr, *rv_wy = nullptr, *rv_wl = nullptr, *rv_wh = nullptr;
     double *rv_tvol = nullptr;                 // the filter's transpose applied to the volumes
     double *adj_gp[2] = {};                    // g_bar of a stage as 9 arrays of pairs (ping-pong)

@@ -627,7 +627,7 @@ namespace {
 // slots; list[t * tsize / 2 ...] the sorted nodes.
 constexpr int kHaloThreads = 256;
 __global__ void __launch_bounds__(kHaloThreads) k_tile_halos(int n, int nslices, const long long *slice_ptr, const int *cnt,
-                                                             const int *lidx, int tsize, int *list, int *count) {
+                                                             const int *lidx, int tslices, int tsize, int *list, int *count) {
     extern __shared__ int hsm[];
     int *table = hsm, *vals = hsm + tsize;
     __shared__ int num;
@@ -637,7 +637,7 @@ __global__ void __launch_bounds__(kHaloThreads) k_tile_halos(int n, int nslices,
     if (tid == 0) num = 0;
     __syncthreads();
     const int shift = 32 - (31 - __clz(tsize));
-    for (int sl = tile * kTileSlices + warp; sl < min(nslices, (tile + 1) * kTileSlices); sl += kHaloThreads / 32) {
+    for (int sl = tile * tslices + warp; sl < min(nslices, (tile + 1) * tslices); sl += kHaloThreads / 32) {
         const int i = sl * kSlice + lane;
         const int c = i < n ? cnt[i] : 0;
         const long long base = slice_ptr[sl];
@@ -694,7 +694,7 @@ __global__ void __launch_bounds__(kHaloThreads) k_tile_halos(int n, int nslices,
 // The tiles' halos into one list, and each link's position in its tile's halo | reflection code
 // << 14 (0 in the padding), by binary search in shared memory.
 __global__ void __launch_bounds__(kHaloThreads) k_halo_links(int n, int nslices, const long long *slice_ptr, const int *slice_w,
-                                                             const int *cnt, const int *lidx, const int *list, int half,
+                                                             const int *cnt, const int *lidx, const int *list, int tslices, int half,
                                                              const int *halo_ptr, int *halo, uint16_t *lloc) {
     extern __shared__ int hsm[];
     const int tile = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -705,7 +705,7 @@ __global__ void __launch_bounds__(kHaloThreads) k_halo_links(int n, int nslices,
         halo[h0 + e] = v;
     }
     __syncthreads();
-    for (int sl = tile * kTileSlices + warp; sl < min(nslices, (tile + 1) * kTileSlices); sl += kHaloThreads / 32) {
+    for (int sl = tile * tslices + warp; sl < min(nslices, (tile + 1) * tslices); sl += kHaloThreads / 32) {
         const int i = sl * kSlice + lane;
         const int c = i < n ? cnt[i] : 0;
         const long long base = slice_ptr[sl];
@@ -733,11 +733,27 @@ __global__ void __launch_bounds__(kHaloThreads) k_halo_links(int n, int nslices,
 
 }  // namespace
 
+// Slices a tile takes; the other warps of its block share the links of the same nodes.  As few
+// as leave the set's tiles at most two a SM: a set that fills the device keeps whole tiles, whose
+// halo is the smallest a node (FP64 step, microseconds with 8, 4, 2 and 1 slices: 4,096 nodes at
+// order 8 100, 71, 58, 50; 16,384 118, 83, 75, 102; 36,864 132, 110, 138, 163; 65,536 178, 227,
+// 214, 265; the cylinder channel's 34,853 159, 123, 141, 155; order 4 at 16,384 55, 43, 42, 61).
+// Mixed precision keeps whole tiles: its FP32 sums in another order, and offsets from other
+// references, change the fields by 1e-9 to 1e-8.
+static int tile_slices(Handle *H, int nslices, int *ts) {
+    int nsm = 0;
+    SUNSET_CUDA(H, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, H->device));
+    *ts = H->cfg.precision == SUNSET_MIXED ? kTileSlices : 1;
+    while (*ts < kTileSlices && nslices > 2 * nsm * *ts) *ts *= 2;
+    return 0;
+}
+
 int build_halos(Handle *H) {
     const int n = H->npfb, nsl = H->nslices;
     const long long L = H->nlinks_sell;
     cudaStream_t st = H->stream;
-    const int nt = (nsl + kTileSlices - 1) / kTileSlices;
+    if (int rc = tile_slices(H, nsl, &H->tslices)) return rc;
+    const int ts = H->tslices, nt = (nsl + ts - 1) / ts;
     // the hash set: 4096 slots hold the halos of the orders' own stencils (2048 nodes a tile);
     // where one is larger, 32768, the most a block's shared memory and the 14-bit index take
     int *list = nullptr, *count = nullptr, tsize = 4096, hmax = 0;
@@ -747,7 +763,7 @@ int build_halos(Handle *H) {
         const int smem = (tsize + tsize / 2) * (int)sizeof(int);
         if (dalloc(H, &list, (size_t)nt * (tsize / 2))) return SUNSET_ERR_NOMEM;
         SUNSET_CUDA(H, cudaFuncSetAttribute(k_tile_halos, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        k_tile_halos<<<nt, kHaloThreads, smem, st>>>(n, nsl, H->slice_ptr, H->cnt, H->lidx, tsize, list, count);
+        k_tile_halos<<<nt, kHaloThreads, smem, st>>>(n, nsl, H->slice_ptr, H->cnt, H->lidx, ts, tsize, list, count);
         SUNSET_CUDA(H, cudaGetLastError());
         SUNSET_CUDA(H, cudaMemcpyAsync(hptr.data() + 1, count, nt * sizeof(int), cudaMemcpyDeviceToHost, st));
         SUNSET_CUDA(H, cudaStreamSynchronize(st));
@@ -771,7 +787,7 @@ int build_halos(Handle *H) {
     SUNSET_CUDA(H, cudaMemcpyAsync(H->halo_ptr, hptr.data(), hptr.size() * sizeof(int), cudaMemcpyHostToDevice, st));
     const int smem = hmax * (int)sizeof(int);
     SUNSET_CUDA(H, cudaFuncSetAttribute(k_halo_links, cudaFuncAttributeMaxDynamicSharedMemorySize, (kLocMask + 1) * (int)sizeof(int)));
-    k_halo_links<<<nt, kHaloThreads, smem, st>>>(n, nsl, H->slice_ptr, H->slice_w, H->cnt, H->lidx, list, tsize / 2,
+    k_halo_links<<<nt, kHaloThreads, smem, st>>>(n, nsl, H->slice_ptr, H->slice_w, H->cnt, H->lidx, list, ts, tsize / 2,
                                                  H->halo_ptr, H->halo, H->lloc);
     SUNSET_CUDA(H, cudaGetLastError());
     SUNSET_CUDA(H, cudaStreamSynchronize(st));

@@ -39,6 +39,7 @@ struct StageArgs {
     const uint16_t *lloc;
     const int *halo_ptr, *halo;
     int hmax;
+    int tslices;  // slices of a tile (kTileSlices unless the set is small)
     const double *wx, *wy, *wl, *wh;
     // mixed precision: the stage's packed links and their per-node scales (stream.cu), the
     // filter's FP32 weights
@@ -173,7 +174,7 @@ __device__ __forceinline__ void load_halo(const StageArgs &A, double *sm, SRC sr
 // indices -- D-1 pairs ahead of the pair it works on, so D-1 pairs per thread are in flight
 // without holding registers.  A thread reads back only what it copied itself, so no barrier
 // is needed; slots are reused only after the thread has consumed them.
-template <bool MX, int NA, int D>
+template <bool MX, int NA, int D, bool SPLIT = false>
 struct LinkRing {
     static_assert((D & (D - 1)) == 0, "ring depth must be a power of two");
     using W2 = typename std::conditional<MX, float2, double2>::type;
@@ -181,22 +182,25 @@ struct LinkRing {
     unsigned *l;    // [D][kTile]
     const W2 *src[NA];
     const unsigned *lsrc;
-    long long pb;   // pair index of this node's pair 0; pair m sits at pb + 32 m
-    int npair;
+    long long pb;   // pair index of this thread's pair 0; pair m sits at pb + 32 m (SPLIT: pb + step m)
+    int npair, step;
 
     static constexpr size_t bytes() { return (size_t)D * kTile * (NA * sizeof(W2) + sizeof(unsigned)); }
 
-    __device__ __forceinline__ void init(double *base, const unsigned *lidx2, long long pb_, int npair_) {
+    // the node's pairs start at pb_ and number npair_; the thread takes pairs part, part + parts, ...
+    __device__ __forceinline__ void init(double *base, const unsigned *lidx2, long long pb_, int npair_, int part = 0,
+                                         int parts = 1) {
         w = reinterpret_cast<W2 *>(base);
         l = reinterpret_cast<unsigned *>(w + (size_t)D * NA * kTile);
         lsrc = lidx2;
-        pb = pb_;
-        npair = npair_;
+        pb = SPLIT ? pb_ + 32 * part : pb_;
+        npair = SPLIT ? (npair_ - part + parts - 1) / parts : npair_;
+        step = 32 * parts;
     }
     __device__ __forceinline__ void issue(int m) {
         if (m < npair) {
             const int s = m & (D - 1);
-            const long long o = pb + ((long long)m << 5);
+            const long long o = SPLIT ? pb + m * step : pb + ((long long)m << 5);
 #pragma unroll
             for (int a = 0; a < NA; a++) cp_async_link<sizeof(W2)>(w + (s * NA + a) * kTile + threadIdx.x, src[a] + o);
             cp_async<4>(l + s * kTile + threadIdx.x, lsrc + o);
@@ -241,14 +245,52 @@ __host__ __device__ constexpr int filter_ring_depth(bool mx) { return mx ? SUNSE
 // Doubles of the shared-memory halo, rounded up so the ring after it is 16-byte aligned.
 __host__ __device__ inline size_t halo_doubles(int ng, int hmax) { return ((size_t)ng * hmax + 1) & ~(size_t)1; }
 
+// Where a block's threads stand.  SPLIT (a small set): kTileSlices / tslices threads share a
+// node's links, and warp w holds part w / tslices of the links of the tile's slice w % tslices.
+struct TilePos {
+    int slice, i, part, parts;
+    bool live;  // the slice exists
+};
+template <bool SPLIT>
+__device__ __forceinline__ TilePos tile_pos(const StageArgs &A) {
+    const int warp = threadIdx.x >> 5;
+    TilePos p;
+    p.parts = SPLIT ? kTileSlices / A.tslices : 1;
+    p.part = SPLIT ? warp / A.tslices : 0;
+    p.slice = SPLIT ? blockIdx.x * A.tslices + warp - p.part * A.tslices : (blockIdx.x * kTile + threadIdx.x) >> 5;
+    p.i = SPLIT ? p.slice * kSlice + (threadIdx.x & 31) : blockIdx.x * kTile + threadIdx.x;
+    p.live = p.slice < A.K.nslices;
+    return p;
+}
+// Adds the parts' sums into part 0's, halving the parts each time; each(fn) applies fn to every
+// sum of the thread.  All threads of the block take part.  buf holds 128 values a sum: it is the
+// link ring's space, which no thread reads any more.
+template <class EACH>
+__device__ __forceinline__ void combine_parts(const StageArgs &A, const TilePos &tp, double *buf, EACH each) {
+    const int part = tp.part;
+    for (int h = tp.parts >> 1; h > 0; h >>= 1) {
+        const int width = h * A.tslices * 32;
+        __syncthreads();
+        if (part >= h && part < 2 * h) {
+            double *b = buf + threadIdx.x - width;
+            each([&](double &x) { *b = x; b += width; });
+        }
+        __syncthreads();
+        if (part < h) {
+            const double *b = buf + threadIdx.x;
+            each([&](double &x) { x = x + *b; b += width; });
+        }
+    }
+}
+
 // Stencil sums of one node over its small links, sum form of derivatives.F90:36-46,
 // neighbours read from the block's shared-memory halo.  In the mixed path the weights are
 // the FP32-rounded ones and A.gsx.. hold the FP64 sums of those, so the FP64 arithmetic
 // below evaluates the difference form sum_k w_k (phi_j - phi_i) of the rounded stencil.
-template <int FORM, bool MD, bool MX, bool FP, class RING>
-__device__ __forceinline__ void gather_stage(const StageArgs &A, int i, const double *sm, RING &R, Grads &g) {
+template <int FORM, bool MD, bool MX, bool FP, bool SPLIT, class RING>
+__device__ __forceinline__ void gather_stage(const StageArgs &A, const TilePos &tp, const double *sm, RING &R, Grads &g) {
     const StepConsts &cK = A.K;
-    const int hm = A.hmax;
+    const int i = tp.i, hm = A.hmax;
     const int npair = R.npair;
     const Fields &F = A.in;
     double s_ro_x = 0, s_ro_y = 0, s_u_x = 0, s_u_y = 0, s_v_x = 0, s_v_y = 0, s_lu = 0, s_lv = 0;
@@ -329,6 +371,21 @@ __device__ __forceinline__ void gather_stage(const StageArgs &A, int i, const do
         const unsigned l2 = R.index(m);
         link((int)(l2 & 0xffffu), wx0, wy0, wl0);
         link((int)(l2 >> 16), wx1, wy1, wl1);
+    }
+    if constexpr (SPLIT) {
+        combine_parts(A, tp, reinterpret_cast<double *>(R.w), [&](auto f) {
+            f(s_ro_x); f(s_ro_y); f(s_u_x); f(s_u_y); f(s_lu); f(s_v_x); f(s_v_y); f(s_lv);
+            if constexpr (FORM == SUNSET_FORM_DI || FORM == SUNSET_FORM_LC) {
+                f(s_cxx_x); f(s_cxy_x); f(s_cxy_y); f(s_cyy_y);
+            }
+            if constexpr (FORM == SUNSET_FORM_DI) { f(s_cxx_y); f(s_cyy_x); }
+            if constexpr (FORM == SUNSET_FORM_LC || FORM == SUNSET_FORM_CHL) {
+                f(s_pxx_x); f(s_pxx_y); f(s_pxy_x); f(s_pxy_y); f(s_pyy_x); f(s_pyy_y);
+            }
+            if constexpr (MD && (FORM == SUNSET_FORM_DI || FORM == SUNSET_FORM_CHL)) { f(s_lxx); f(s_lxy); f(s_lyy); }
+            if constexpr (FP && FORM != SUNSET_FORM_NEWT) { f(s_f_x); f(s_f_y); f(s_lzz); }
+        });
+        if (tp.part) return;
     }
     if (i >= cK.npfb) return;
     const double gx = A.gsx[i], gy = A.gsy[i], ls = A.lsum[i];
@@ -764,13 +821,15 @@ __host__ __device__ constexpr int stage_min_blocks(bool mx) { return mx ? SUNSET
 // O(dt rhs) quantity) and the error accumulator E as FP32.
 // BND: the node set has boundary nodes (walls, inflows, outflows); without them the
 // closures are compiled out, which keeps them from costing the periodic sets registers.
-template <int FORM, bool MD, bool MX, bool FP, bool BND>
+template <int FORM, bool MD, bool MX, bool FP, bool BND, bool SPLIT>
 __global__ void __launch_bounds__(kTile, stage_min_blocks(MX)) k_stage(StageArgs A) {
+    static_assert(!(MX && SPLIT), "the mixed path keeps whole tiles: another order of its FP32 sums shows in the results");
     const StepConsts &cK = A.K;
     extern __shared__ __align__(16) double smem[];
     constexpr int NG = ngather(FORM, MD, FP);
-    const int i = blockIdx.x * kTile + threadIdx.x;
-    bool active = (i >> 5) < cK.nslices;
+    const TilePos tp = tile_pos<SPLIT>(A);
+    const int i = tp.i;
+    bool active = tp.live;
     const int stage = A.stage;
     if (stage == 0 && i == 0) {
         A.sc->cfl_bits = 0x7ff0000000000000ull;
@@ -778,7 +837,7 @@ __global__ void __launch_bounds__(kTile, stage_min_blocks(MX)) k_stage(StageArgs
     }
     Grads g;
     if constexpr (MX) {
-        const int warp = threadIdx.x >> 5, sl = blockIdx.x * kTileSlices + warp;
+        const int warp = threadIdx.x >> 5, sl = tp.slice;
         MxRing R;
         R.ring = reinterpret_cast<uint2 *>(smem) + (size_t)warp * kMxDepth * 3 * kMxChunk * 32;
         R.bar0 = smem_addr(reinterpret_cast<char *>(smem) + mx_ring_bytes() + (size_t)warp * kMxDepth * 8);
@@ -790,15 +849,15 @@ __global__ void __launch_bounds__(kTile, stage_min_blocks(MX)) k_stage(StageArgs
         if (cK.has_mirrors) gather_stage_mx<FORM, MD, FP, true>(A, i, smem, R, active, oi, g);
         else gather_stage_mx<FORM, MD, FP, false>(A, i, smem, R, active, oi, g);
     } else {
-        LinkRing<false, 3, ring_depth(false)> R;
+        LinkRing<false, 3, ring_depth(false), SPLIT> R;
         R.src[0] = reinterpret_cast<const double2 *>(A.wx);
         R.src[1] = reinterpret_cast<const double2 *>(A.wy);
         R.src[2] = reinterpret_cast<const double2 *>(A.wl);
         R.init(smem + halo_doubles(NG, A.hmax), reinterpret_cast<const unsigned *>(A.lloc),
-               active ? (A.slice_ptr[i >> 5] >> 1) + (i & 31) : 0, active ? A.slice_ws[i >> 5] >> 1 : 0);
+               active ? (A.slice_ptr[i >> 5] >> 1) + (i & 31) : 0, active ? A.slice_ws[i >> 5] >> 1 : 0, tp.part, tp.parts);
         R.prologue();  // the first link pairs stream in while the halo is staged
         load_halo<NG>(A, smem, [&](int f) { return gather_src<FORM, MD, FP>(A.in, f); });
-        if (active) gather_stage<FORM, MD, false, FP>(A, i, smem, R, g);
+        if (SPLIT || active) gather_stage<FORM, MD, false, FP, SPLIT>(A, tp, smem, R, g);
     }
     // a node's own value of gathered field f in the tile's halo slot h (wall Laplacian of c)
     auto hv = [&](int f, int h) -> double {
@@ -809,7 +868,7 @@ __global__ void __launch_bounds__(kTile, stage_min_blocks(MX)) k_stage(StageArgs
             return smem[f * A.hmax + h];
         }
     };
-    active = active && i < cK.npfb;
+    active = active && i < cK.npfb && (!SPLIT || tp.part == 0);
     unsigned long long emax_bits = 0;
     if constexpr (FORM == SUNSET_FORM_LC && !MX) {
         if (active && A.gsave) {
@@ -982,20 +1041,20 @@ __global__ void __launch_bounds__(kTile, stage_min_blocks(MX)) k_stage(StageArgs
 // FP (Cholesky FENE-P): psizz is filtered too, and the psi factors of J = f c are converted to
 // factors of c before filtering and back after it (rhs.F90:815-869) -- in shared memory for
 // the halo, in registers for the node itself.
-template <int FORM, bool MX, bool FP = false>
+template <int FORM, bool FP, bool SPLIT>
 __global__ void __launch_bounds__(kTile, 4) k_filter(StageArgs A) {
     const StepConsts &cK = A.K;
     extern __shared__ __align__(16) double smem[];
     constexpr bool CF = FP && FORM == SUNSET_FORM_CHL;
     constexpr int nf = (FORM == SUNSET_FORM_DI || CF) ? 7 : (FORM == SUNSET_FORM_NEWT ? 3 : 6);
     const Fields &F = A.in;
-    const int i = blockIdx.x * kTile + threadIdx.x;
-    const bool live = (i >> 5) < cK.nslices;
-    LinkRing<MX, 1, filter_ring_depth(MX)> R;
-    static_assert(!MX, "the mixed filter is k_filter_mx");
+    const TilePos tp = tile_pos<SPLIT>(A);
+    const int i = tp.i;
+    const bool live = tp.live;
+    LinkRing<false, 1, filter_ring_depth(false), SPLIT> R;
     R.src[0] = reinterpret_cast<const double2 *>(A.wh);
     R.init(smem + halo_doubles(nf, A.hmax), reinterpret_cast<const unsigned *>(A.lloc),
-           live ? (A.slice_ptr[i >> 5] >> 1) + (i & 31) : 0, live ? A.slice_w[i >> 5] >> 1 : 0);
+           live ? (A.slice_ptr[i >> 5] >> 1) + (i & 31) : 0, live ? A.slice_w[i >> 5] >> 1 : 0, tp.part, tp.parts);
     R.prologue();
     load_halo<nf>(A, smem, [&](int f) -> const double * {
         return f == 0 ? F.ro : f == 1 ? F.rou : f == 2 ? F.rov : F.q[f - 3];
@@ -1008,7 +1067,7 @@ __global__ void __launch_bounds__(kTile, 4) k_filter(StageArgs A) {
         __syncthreads();
     }
     double part = 0.0;
-    if (live) {
+    if (SPLIT || live) {
         const int npair = R.npair;
         double t[7] = {0, 0, 0, 0, 0, 0, 0};
         const bool mir = cK.has_mirrors;
@@ -1024,8 +1083,7 @@ __global__ void __launch_bounds__(kTile, 4) k_filter(StageArgs A) {
             }
 #pragma unroll
             for (int f = 0; f < nf; f++) {
-                if constexpr (MX) t[f] = __fma_rn(v[f], whk, t[f]);
-                else t[f] = t[f] + v[f] * whk;
+                t[f] = t[f] + v[f] * whk;
             }
         };
         for (int m = 0; m < npair; m++) {
@@ -1036,7 +1094,12 @@ __global__ void __launch_bounds__(kTile, 4) k_filter(StageArgs A) {
             link((int)(l2 & 0xffffu), wh0);
             link((int)(l2 >> 16), wh1);
         }
-        if (i < cK.npfb) {
+        if constexpr (SPLIT)
+            combine_parts(A, tp, reinterpret_cast<double *>(R.w), [&](auto f) {
+#pragma unroll
+                for (int q = 0; q < nf; q++) f(t[q]);
+            });
+        if (i < cK.npfb && (!SPLIT || tp.part == 0)) {
             const double hs = A.hsum[i];
             const double *src[7] = {F.ro, F.rou, F.rov, F.q[0], F.q[1], F.q[2], F.q[3]};
             double *dst[7] = {A.out.ro, A.out.rou, A.out.rov, A.out.q[0], A.out.q[1], A.out.q[2], A.out.q[3]};
@@ -1643,6 +1706,7 @@ StageArgs make_args(Handle *H, int from, int stage, bool step = false) {
     A.halo_ptr = H->halo_ptr;
     A.halo = H->halo;
     A.hmax = H->halo_max;
+    A.tslices = H->tslices;
     if (step) {
         A.wx = H->wx_s; A.wy = H->wy_s; A.wl = H->wl_s; A.wh = H->wh_s;
     } else {
@@ -1688,17 +1752,20 @@ constexpr size_t kMaxStageSmem = 200 * 1024;
 template <int FORM, bool MD, bool FP>
 int stage_smem_attributes(Handle *H, bool mx) {
     if (H->nb > 0) {
-        SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, true>));
-        if (mx) SUNSET_SMEM_ATTR((k_stage<FORM, MD, true, FP, true>));
+        SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, true, false>));
+        SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, true, true>));
+        if (mx) SUNSET_SMEM_ATTR((k_stage<FORM, MD, true, FP, true, false>));
     } else {
-        SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, false>));
-        if (mx) SUNSET_SMEM_ATTR((k_stage<FORM, MD, true, FP, false>));
+        SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, false, false>));
+        SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, false, true>));
+        if (mx) SUNSET_SMEM_ATTR((k_stage<FORM, MD, true, FP, false, false>));
     }
     return 0;
 }
 template <int FORM, bool FP>
 int filter_smem_attributes(Handle *H, bool mx) {
-    SUNSET_SMEM_ATTR((k_filter<FORM, false, FP>));
+    SUNSET_SMEM_ATTR((k_filter<FORM, FP, false>));
+    SUNSET_SMEM_ATTR((k_filter<FORM, FP, true>));
     if (mx) SUNSET_SMEM_ATTR((k_filter_mx<FORM, FP, true>));
     if (mx) SUNSET_SMEM_ATTR((k_filter_mx<FORM, FP, false>));
     return 0;
@@ -1739,12 +1806,17 @@ int launch_stage(Handle *H, const StageArgs &A, bool mx) {
                            : halo_doubles(ngather(FORM, MD, FP), H->halo_max) * sizeof(double) +
                                  LinkRing<false, 3, ring_depth(false)>::bytes();
     if (smem > kMaxStageSmem) return set_err(H, SUNSET_ERR_SCOPE, "tile halo too large for shared memory");
-    if (H->nb > 0) {
-        if (mx) k_stage<FORM, MD, true, FP, true><<<H->ntiles, kTile, smem, H->stream>>>(A);
-        else k_stage<FORM, MD, false, FP, true><<<H->ntiles, kTile, smem, H->stream>>>(A);
+    const bool bnd = H->nb > 0, split = H->tslices < kTileSlices;
+    auto go = [&](auto kernel) { kernel<<<H->ntiles, kTile, smem, H->stream>>>(A); };
+    if (mx) {
+        if (bnd) go(k_stage<FORM, MD, true, FP, true, false>);
+        else go(k_stage<FORM, MD, true, FP, false, false>);
+    } else if (split) {
+        if (bnd) go(k_stage<FORM, MD, false, FP, true, true>);
+        else go(k_stage<FORM, MD, false, FP, false, true>);
     } else {
-        if (mx) k_stage<FORM, MD, true, FP, false><<<H->ntiles, kTile, smem, H->stream>>>(A);
-        else k_stage<FORM, MD, false, FP, false><<<H->ntiles, kTile, smem, H->stream>>>(A);
+        if (bnd) go(k_stage<FORM, MD, false, FP, true, false>);
+        else go(k_stage<FORM, MD, false, FP, false, false>);
     }
     return 0;
 }
@@ -1783,8 +1855,10 @@ int launch_filter(Handle *H, const StageArgs &A, bool mx) {
     }
     const size_t smem = halo_doubles(nf, H->halo_max) * sizeof(double) + LinkRing<false, 1, filter_ring_depth(false)>::bytes();
     if (smem > kMaxStageSmem) return set_err(H, SUNSET_ERR_SCOPE, "tile halo too large for shared memory");
-    if (cf) k_filter<FORM, false, true><<<H->ntiles, kTile, smem, H->stream>>>(A);
-    else k_filter<FORM, false><<<H->ntiles, kTile, smem, H->stream>>>(A);
+    const bool split = H->tslices < kTileSlices;
+    auto go = [&](auto kernel) { kernel<<<H->ntiles, kTile, smem, H->stream>>>(A); };
+    if (cf) split ? go(k_filter<FORM, true, true>) : go(k_filter<FORM, true, false>);
+    else split ? go(k_filter<FORM, false, true>) : go(k_filter<FORM, false, false>);
     return 0;
 }
 
@@ -1883,7 +1957,8 @@ int state_alloc(Handle *H) {
     if (H->nb > 0 && dalloc(H, &H->uin, H->nb)) return SUNSET_ERR_NOMEM;
     const int nthr = H->nslices * kSlice;
     H->npart = (nthr + 127) / 128 + 1;
-    if (dalloc(H, &H->partials, 2 * (size_t)H->npart + 16) || dalloc(H, &H->dsc, 1) || dalloc(H, &H->tmpd, 4 * (size_t)n))
+    // block sums of the reductions: two a block of 128 nodes, or one a tile
+    if (dalloc(H, &H->partials, std::max(2 * (size_t)H->npart, (size_t)H->ntiles) + 16) || dalloc(H, &H->dsc, 1) || dalloc(H, &H->tmpd, 4 * (size_t)n))
         return SUNSET_ERR_NOMEM;
     SUNSET_CUDA(H, cudaMemsetAsync(H->dsc, 0, sizeof(DevScalars), H->stream));
     return 0;
@@ -2811,6 +2886,7 @@ static int adjoint_build_stream(Handle *H) {
     SUNSET_CUDA(H, cudaMemcpyAsync(dslot, slot_s.data(), L * sizeof(int), cudaMemcpyHostToDevice, H->stream));
     SUNSET_CUDA(H, cudaMemcpyAsync(dslot + Lz, slot_f.data(), L * sizeof(int), cudaMemcpyHostToDevice, H->stream));
     H->rv_hmax = hmax;
+    H->rv_ntiles = nt;
     if (L)
         k_adj_stream_weights<<<(unsigned)((L + 255) / 256), 256, 0, H->stream>>>(
             L, dslot, dslot + Lz, H->wx, H->wy, H->wl, H->wh, H->rv_wx, H->rv_wy, H->rv_wl, H->rv_wh);
@@ -2918,7 +2994,7 @@ int adjoint_run(Handle *H, double dt, int nsteps, int ckpt, double *J, double *d
             if (dalloc(H, &H->adj_sb[k], n) || dalloc(H, &H->adj_sbar[k], n)) return SUNSET_ERR_NOMEM;
         for (int f = 0; f < 7; f++)
             if (dalloc(H, &H->adj_ua[f], n)) return SUNSET_ERR_NOMEM;
-        if (dalloc(H, &H->adj_tacc, 2 * (size_t)H->ntiles) || dalloc(H, &H->adj_rpart, (size_t)H->ntiles) ||
+        if (dalloc(H, &H->adj_tacc, 2 * (size_t)H->rv_ntiles) || dalloc(H, &H->adj_rpart, (size_t)H->rv_ntiles) ||
             dalloc(H, &H->adj_acc, 4))
             return SUNSET_ERR_NOMEM;
         SUNSET_CUDA(H, cudaFuncSetAttribute(k_adj_stage_lc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxStageSmem));
@@ -3001,8 +3077,8 @@ int adjoint_run(Handle *H, double dt, int nsteps, int ckpt, double *J, double *d
     // ---- reverse ----
     RevArgs B = rev_args(H);
     B.dt = dt;
-    k_adj_objective<<<H->ntiles, kTile, 0, st>>>(H->buf[H->cur], H->vol, B);
-    SUNSET_CUDA(H, cudaMemsetAsync(H->adj_tacc, 0, 2 * (size_t)H->ntiles * sizeof(double), st));
+    k_adj_objective<<<H->rv_ntiles, kTile, 0, st>>>(H->buf[H->cur], H->vol, B);
+    SUNSET_CUDA(H, cudaMemsetAsync(H->adj_tacc, 0, 2 * (size_t)H->rv_ntiles * sizeof(double), st));
     const double alpha[4] = {SUNSET_RK_A21, SUNSET_RK_A32, SUNSET_RK_A43, SUNSET_RK_B4};
     const double beta[4] = {SUNSET_RK_B1, SUNSET_RK_B2, SUNSET_RK_B3, 0.0};
     auto gstage = [&](int k, int s) { return H->adj_g + (size_t)(4 * k + s) * kAdjG * n; };
@@ -3018,7 +3094,7 @@ int adjoint_run(Handle *H, double dt, int nsteps, int ckpt, double *J, double *d
             B.alpha = alpha[3];
             B.beta = beta[3];
             B.first = 0;
-            k_adj_filter_lc<<<H->ntiles, kTile, smem_filter, st>>>(B);
+            k_adj_filter_lc<<<H->rv_ntiles, kTile, smem_filter, st>>>(B);
             int cur = 0;
             for (int s = 3; s >= 1; s--) {  // stencils of stage s, pointwise reverse of stage s - 1
                 B.cur = H->adj_store[4 * k + s];
@@ -3029,12 +3105,12 @@ int adjoint_run(Handle *H, double dt, int nsteps, int ckpt, double *J, double *d
                 B.alpha = alpha[s - 1];
                 B.beta = beta[s - 1];
                 B.first = first && (s == 1) && (sc0.itime + n0 + k == 1);
-                k_adj_stage_lc<true><<<H->ntiles, kTile, smem_stage, st>>>(B);
+                k_adj_stage_lc<true><<<H->rv_ntiles, kTile, smem_stage, st>>>(B);
                 cur ^= 1;
             }
             B.cur = H->adj_store[4 * k];
             B.gb_in = gpair(cur);
-            k_adj_stage_lc<false><<<H->ntiles, kTile, smem_stage, st>>>(B);
+            k_adj_stage_lc<false><<<H->rv_ntiles, kTile, smem_stage, st>>>(B);
         }
         SUNSET_CUDA(H, cudaGetLastError());
         return 0;
@@ -3053,7 +3129,7 @@ int adjoint_run(Handle *H, double dt, int nsteps, int ckpt, double *J, double *d
         SUNSET_CUDA(H, cudaGraphLaunch(H->adj_rev_graph, st));
     }
     SUNSET_CUDA(H, cudaGetLastError());
-    k_adj_fold<<<1, 128, 0, st>>>(H->adj_tacc, H->ntiles, 2, H->adj_acc, 0);
+    k_adj_fold<<<1, 128, 0, st>>>(H->adj_tacc, H->rv_ntiles, 2, H->adj_acc, 0);
     double acc[2];
     SUNSET_CUDA(H, cudaMemcpyAsync(acc, H->adj_acc, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
     for (int f = 0; f < kAdjS; f++)

@@ -1,6 +1,7 @@
 """The set-up kernels at the sizes where they can go wrong: the device's bank-aware link order
-against the host's, the weight build over several batches and at order 10, and the tile halos
-of a stencil too wide for the smaller hash set.
+against the host's, the weight build over several batches and at order 10, the tile halos of a
+stencil too wide for the smaller hash set, and the tiles of small sets, whose nodes' links
+several threads share.
 
 The link order is compared entry by entry; the weights bit for bit with the restatement (both
 round every operation alike, with its correctly rounded x^4), except the filter's, which CUDA's
@@ -84,3 +85,34 @@ def test_wide_stencil_halos():
     # the largest term: the viscous force, (1 / s^2) |u|, and the pressure gradient, c^2 |grad rho|
     for k in ("ro", "rou", "rov", "xx", "xy", "yy"):
         assert np.abs(a[k] - b[k]).max() <= 1e-10 * max(1.0, np.abs(b[k]).max()), k
+
+
+# 2 n_SM = 296 tiles at most: tiles of 1, 1 (the largest such set), 2, 4 and 8 slices on 148 SMs
+@pytest.mark.parametrize("form,order", [("di", 4), ("lc", 4), ("chl", 6)])
+@pytest.mark.parametrize("nside", [17, 97, 98, 150, 201])
+def test_small_set_tiles(nside, form, order):
+    ns = jittered_lattice(nside)
+    O.set_pow_mode(True)
+    try:
+        ref = O.Oracle(form=form, order=order, h_over_s={4: 1.5, 6: 2.1}[order]).build_domain(ns).setup()
+    finally:
+        O.set_pow_mode(False)
+    gpus = [labfm.Sunset(form=form, order=order, h_over_s={4: 1.5, 6: 2.1}[order], precision=p).build_domain(ns).setup()
+            for p in ("fp64", "mixed")]
+    st = initial_state(ns)
+    st["ro"] = 1.0 + 0.01 * np.cos(2 * np.pi * ns.x)
+    st["cxx"] = 1.3 + 0.2 * np.sin(2 * np.pi * ns.x)
+    st["cxy"] = 0.1 * np.cos(2 * np.pi * ns.y)
+    for g in [ref] + gpus:
+        g.set_state(**st)
+    a, b = gpus[0].rhs(), ref.rhs()
+    for k in ("ro", "rou", "rov", "xx", "xy", "yy"):
+        assert np.abs(a[k] - b[k]).max() <= 1e-10 * max(1.0, np.abs(b[k]).max()), k
+    dt = 0.1 / (nside * nside)
+    for g in [ref] + gpus:
+        g.step(dt, 3)
+    want = ref.state()
+    for g, tol in zip(gpus, (1e-10, 1e-6)):  # mixed: the tolerance its fields keep over 100 steps
+        got = g.state()
+        for k in ("ro", "u", "v", "cxx", "cxy", "cyy"):
+            assert np.abs(got[k] - want[k]).max() <= tol * max(1.0, np.abs(want[k]).max()), k
