@@ -737,13 +737,18 @@ __global__ void __launch_bounds__(kHaloThreads) k_halo_links(int n, int nslices,
 // as leave the set's tiles at most two a SM: a set that fills the device keeps whole tiles, whose
 // halo is the smallest a node (FP64 step, microseconds with 8, 4, 2 and 1 slices: 4,096 nodes at
 // order 8 100, 71, 58, 50; 16,384 118, 83, 75, 102; 36,864 132, 110, 138, 163; 65,536 178, 227,
-// 214, 265; the cylinder channel's 34,853 159, 123, 141, 155; order 4 at 16,384 55, 43, 42, 61).
-// Mixed precision keeps whole tiles: its FP32 sums in another order, and offsets from other
-// references, change the fields by 1e-9 to 1e-8.
+// 214, 265; order 4 at 16,384 55, 43, 42, 61).
+//
+// Shared links are summed in another order.  That is rounding on the periodic sets (3e-16), but
+// the sets with boundary nodes can hold a stencil that amplifies it (the cylinder channel: 3e-8
+// of the momentum after twenty steps on some seeds), and in mixed precision FP32 sums in
+// another order, from other offsets, change the fields by 1e-9 to 3e-8: both keep whole tiles.
+// Two ways that keep the order gained too little: a thread a node in smaller blocks with rings
+// eight deep (4,096 nodes 96 -> 90), a warp a gathered field (95 -> 86, and 115 -> 156 at 16,384).
 static int tile_slices(Handle *H, int nslices, int *ts) {
     int nsm = 0;
     SUNSET_CUDA(H, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, H->device));
-    *ts = H->cfg.precision == SUNSET_MIXED ? kTileSlices : 1;
+    *ts = H->cfg.precision == SUNSET_MIXED || H->nb > 0 ? kTileSlices : 1;
     while (*ts < kTileSlices && nslices > 2 * nsm * *ts) *ts *= 2;
     return 0;
 }
