@@ -8,13 +8,14 @@
 // update, rows of a Givens rotation), and every dot product is summed by one thread in the
 // reference's order.  With -fmad=false each operation then rounds exactly as the
 // reference's does, so the factorisation - and the weights - are those of the CPU
-// restatement bit for bit.  The weight build takes three kernels (below); the stencil
-// adaptation and the boundary operators factor on one warp (svd_factor_warp).
+// restatement bit for bit.  The weight build takes three kernels (below), the stencil
+// adaptation a block a node, and the boundary operators factor on one warp (svd_factor_warp).
 //
 // The five SVDs of identical matrix copies in labf.F90:157-180 become one factorisation
 // applied to five right-hand sides; the filter matrix (labf.F90:258-303) is the same
 // matrix whenever h == h_small, the counts agree and the order drops agree, and is then
 // not factored again.
+#include <algorithm>
 #include <cmath>
 
 #include "internal.cuh"
@@ -70,24 +71,6 @@ __device__ __forceinline__ double hermite(int n, double z) {
         return ((((((z4 * z4) * z2) - ((45.0 * z4) * z4)) + ((630.0 * z4) * z2)) - (3150.0 * z4)) + (4725.0 * z2)) - 945.0;
     }
     return 0.0;
-}
-
-// x^p y^q / (p! q!) as written in labf.F90:1815-1920: x2=x*x, x3=x2*x, ..., then
-// (coef*x^p)*y^q.
-__device__ __forceinline__ double monomial(int p, int q, double x, double y) {
-    double xp = x, yq = y;
-    for (int k = 2; k <= p; k++) xp = xp * x;
-    for (int k = 2; k <= q; k++) yq = yq * y;
-    double den = fact(p) * fact(q);
-    if (den == 1.0) {
-        if (p == 0) return yq;
-        if (q == 0) return xp;
-        return xp * yq;
-    }
-    double c = 1.0 / den;
-    if (q == 0) return c * xp;
-    if (p == 0) return c * yq;
-    return (c * xp) * yq;
 }
 
 // x^4 correctly rounded.  The reference evaluates (1-q/2)**4.0 with libm pow; glibc's pow
@@ -385,37 +368,6 @@ __device__ __forceinline__ long long sell_off(const long long *slice_ptr, int i,
     return sell_at(slice_ptr[i >> 5], k, i & 31);
 }
 
-// Moment matrix over links [0,cnt) of node i with length scale hh (labf.F90:88-123).
-template <int ORDER>
-__device__ void assemble(const WArgs &a, int i, int cnt, double hh, double *U, int ld, double *X, double *G,
-                         int lane) {
-    constexpr int n = nsz(ORDER);
-    __syncwarp();
-    for (int e = lane; e < n * n; e += 32) U[(e / n) * ld + (e % n)] = 0.0;
-    const double xi = a.px[i], yi = a.py[i];
-    for (int k = 0; k < cnt; k++) {
-        int p = a.lpt[sell_off(a.slice_ptr, i, k)];
-        double x = -(xi - a.px[p]), y = -(yi - a.py[p]);
-        double rad = sqrt(x * x + y * y) / hh;
-        double ff1 = wab(rad, a.h2);
-        double xx = x / hh, yy = y / hh;
-        __syncwarp();
-        for (int m = lane; m < n; m += 32) {
-            int pm = p_of(m), qm = q_of(m);
-            X[m] = monomial(pm, qm, x / hh, y / hh);
-            double g = (qm == 0) ? hermite(pm, xx) : (pm == 0) ? hermite(qm, yy) : hermite(pm, xx) * hermite(qm, yy);
-            G[m] = g * ff1;
-        }
-        __syncwarp();
-        for (int e = lane; e < n * n; e += 32) {
-            int i1 = e % n, i2 = e / n;
-            double *u = &U[i2 * ld + i1];
-            *u = *u + X[i1] * G[i2];
-        }
-    }
-    __syncwarp();
-}
-
 // ---------------------------------------------------------------------------------------
 // The weight build in three kernels over batches of nodes.
 //
@@ -505,25 +457,24 @@ __global__ void k_weight_items(WArgs a, int *item0, int *item1, int *count) {
     if (!same_matrix(a, i, t)) item1[atomicAdd(&count[1], 1)] = i;
 }
 
-// Moment matrix (labf.F90:88-148 or 258-303) and svdlib.F90:37-171 of one node a block.
-// Bound: the FP64 sums in the reference's serial order (a column's dot product is one chain),
-// seven blocks of two warps a SM at order 8 (32 KB of shared memory each).
+// A block's moment matrix over links [0, cnt) with length hh (labf.F90:88-148 or 258-303; only the
+// first `keep` unknowns, the identity beyond) and svdlib.F90:37-171: on return U and V are the
+// accumulated transformations (column-major, leading dimension n | 1) and W, rv1 (1-based) the
+// bidiagonal, all in shared memory (bidiag_doubles of it at smem, U first); returns anorm.  M, if
+// not null, gets the matrix.  Bound: the FP64 sums in the reference's serial order (a
+// column's dot product is one chain), six blocks of two warps a SM at order 8.
 template <int ORDER>
-__global__ void __launch_bounds__(bidiag_threads(ORDER)) k_moment_bidiag(WArgs a, SvdBatch B) {
+__device__ double moment_bidiag(const WArgs &a, int i0, int cnt, double hh, int keep, double *smem, double *U, double *V,
+                                double *W, double *rv1, double *M) {
     constexpr int n = nsz(ORDER), ld = n | 1, T = bidiag_threads(ORDER);
-    extern __shared__ double smem[];
-    const int it = blockIdx.x, tid = threadIdx.x;
-    const int i0 = B.item[it], t = a.ntype[i0];
-    double *U = smem, *V = U + n * ld;
-    double *rv1 = smem + bidiag_doubles<ORDER>() - 2 * (n + 2), *W = rv1 + (n + 2);
+    const int tid = threadIdx.x;
     auto sync = [] {
         if constexpr (T == 32) __syncwarp();
         else __syncthreads();
     };
-    const double hh = B.pass ? a.h[i0] : a.hs[i0];
-    const int cnt = B.pass ? a.cnt[i0] : a.cnt_small[i0];
     {
-        // the thread's unknown: exponents and 1 / (p! q!) of its monomial (see monomial())
+        // the thread's unknown: exponents and 1 / (p! q!) of its monomial x^p y^q / (p! q!), evaluated
+        // as written in labf.F90:1815-1920: x2=x*x, x3=x2*x, ..., then (coef*x^p)*y^q
         const int m = tid < n ? tid : 0;
         const int pm = p_of(m), qm = q_of(m);
         const double den = fact(pm) * fact(qm), inv = 1.0 / den;
@@ -576,18 +527,13 @@ __global__ void __launch_bounds__(bidiag_threads(ORDER)) k_moment_bidiag(WArgs a
             }
         }
         sync();
-        // labf.F90:125-148, 305-323: next to walls only the first unknowns are kept
-        int keep = n;
-        if (B.pass == 0) {
-            if (a.morder >= 7 && (t == 998 || t < 0)) keep = min(keep, 27);
-            if (a.morder >= 5 && (t == -1 || t == -2)) keep = min(keep, 14);
-        } else {
-            if (a.forder >= 7 && (t == 998 || t < 0)) keep = min(keep, 27);
-            if (a.forder >= 5 && t == -1) keep = min(keep, 14);
-        }
         if (tid < n) {
 #pragma unroll
             for (int r = 0; r < n; r++) U[tid * ld + r] = (tid >= keep || r >= keep) ? (r == tid ? 1.0 : 0.0) : acc[r];
+            if (M) {
+#pragma unroll
+                for (int r = 0; r < n; r++) M[tid * ld + r] = acc[r];
+            }
         }
         sync();
     }
@@ -708,6 +654,31 @@ __global__ void __launch_bounds__(bidiag_threads(ORDER)) k_moment_bidiag(WArgs a
         }
         sync();
     }
+    return anorm;
+#undef UM
+#undef VM
+}
+
+// One item a block: its matrix and the batch's arrays.
+template <int ORDER>
+__global__ void __launch_bounds__(bidiag_threads(ORDER)) k_moment_bidiag(WArgs a, SvdBatch B) {
+    constexpr int n = nsz(ORDER), ld = n | 1, T = bidiag_threads(ORDER);
+    extern __shared__ double smem[];
+    const int it = blockIdx.x, tid = threadIdx.x, me = tid + 1;
+    const int i0 = B.item[it], t = a.ntype[i0];
+    double *U = smem, *V = U + n * ld;
+    double *rv1 = smem + bidiag_doubles<ORDER>() - 2 * (n + 2), *W = rv1 + (n + 2);
+    // labf.F90:125-148, 305-323: next to walls only the first unknowns are kept
+    int keep = n;
+    if (B.pass == 0) {
+        if (a.morder >= 7 && (t == 998 || t < 0)) keep = min(keep, 27);
+        if (a.morder >= 5 && (t == -1 || t == -2)) keep = min(keep, 14);
+    } else {
+        if (a.forder >= 7 && (t == 998 || t < 0)) keep = min(keep, 27);
+        if (a.forder >= 5 && t == -1) keep = min(keep, 14);
+    }
+    const double anorm = moment_bidiag<ORDER>(a, i0, B.pass ? a.cnt[i0] : a.cnt_small[i0], B.pass ? a.h[i0] : a.hs[i0], keep,
+                                              smem, U, V, W, rv1, nullptr);
     // the rows of U that the solves read, V, and the bidiagonal
     const int fo = filter_order(a.forder, t);
     for (int e = tid; e < kUrows * n; e += T) {
@@ -726,8 +697,6 @@ __global__ void __launch_bounds__(bidiag_threads(ORDER)) k_moment_bidiag(WArgs a
         B.anorm[it] = anorm;
         B.state[it] = make_int2(n, 1);
     }
-#undef UM
-#undef VM
 }
 
 // What a record entry's header says the entries after it are.
@@ -1486,36 +1455,174 @@ __global__ void k_boundary_frame(BndArgs a) {
 // `limit` reductions have been made.  Pass 0 reduces h (h_small with it) over the node's
 // list, pass 1 h_small over its small list.  The lists are sorted by distance, so the links
 // within 2 h are a prefix of each.  The arithmetic follows the CPU restatement operation for
-// operation (the same moment matrix, warp SVD and sums in the same order); the amplification
-// sums run one wavenumber per lane, each over the links in order.  A moment matrix whose SVD
+// operation (the same moment matrix, SVD and sums in the same order); the amplification
+// sums run one wavenumber a thread, each over the links in order.  A moment matrix whose SVD
 // does not converge ends the node's reduction (the reference stops).
 struct AdaptArgs {
     WArgs w;
     double *h, *hs;
     const double *sp;
-    int nplink, per_warp;
+    double *M;  // a moment matrix a block
+    int *next;  // the next node to take
+    int nplink;
     double rf, limit, res_tol[2];
 };
 
+// Rows of U that the three solves read: 0, 1, 2 and 4.
+constexpr int kAdaptUrows = 4;
 template <int ORDER>
-__host__ __device__ constexpr int adapt_fixed_doubles() {
-    return 2 * nsz(ORDER) * (nsz(ORDER) | 1) + 3 * (nsz(ORDER) + 2) + nsz(ORDER) * (nsz(ORDER) | 1) + 6 * nsz(ORDER);
+__host__ __device__ constexpr int adapt_vectors() {  // the warps' bidiagonals, tmp, bl, bx, by, residual
+    return (bidiag_threads(ORDER) / 32) * 2 * (nsz(ORDER) + 2) + 5 * nsz(ORDER) + 8;
+}
+// The links' coordinates and dot products take the place of U and V, which are used up by then.
+template <int ORDER>
+__host__ __device__ inline int adapt_doubles(int nplink) {
+    const int mats = bidiag_doubles<ORDER>(), links = 5 * nplink;
+    return (mats > links ? mats : links) + adapt_vectors<ORDER>();
 }
 
+// One node a block at a time.  Every length tried takes a factorisation: the block function
+// above, then the QR iteration, whose scalars every warp carries along by itself (its own copy
+// of the bidiagonal) while each thread turns one row of V, or of the four rows of U that the
+// solves read.  One warp a node with all of U, V and the matrix in shared memory held four
+// nodes a SM and took 1.5 ms a factorisation at order 8.
 template <int ORDER>
-__global__ void k_adapt_stencils(AdaptArgs a) {
-    constexpr int n = nsz(ORDER);
-    constexpr int ld = n | 1;
+__global__ void __launch_bounds__(bidiag_threads(ORDER)) k_adapt_stencils(AdaptArgs a) {
+    constexpr int n = nsz(ORDER), ld = n | 1, T = bidiag_threads(ORDER);
+    static_assert(n + kAdaptUrows <= T, "a thread a row");
     extern __shared__ double smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-    double *U = smem + (size_t)warp * a.per_warp;
-    double *V = U + n * ld, *W = V + n * ld, *rv1 = W + (n + 2), *tmp = rv1 + (n + 2), *M = tmp + (n + 2);
-    double *X = M + n * ld, *G = X + n, *bl = G + n, *bx = bl + n, *by = bx + n, *R = by + n;
-    double *lx = R + n, *ly = lx + a.nplink, *dl = ly + a.nplink, *dxv = dl + a.nplink, *dyv = dxv + a.nplink;
+    __shared__ int sh_i, sh_cnt, sh_bad;
+    __shared__ double sh_hc;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    auto sync = [] {
+        if constexpr (T == 32) __syncwarp();
+        else __syncthreads();
+    };
+    double *U = smem, *V = U + n * ld;
+    double *rv1 = smem + bidiag_doubles<ORDER>() - 2 * (n + 2), *W = rv1 + (n + 2);
+    const int mats = bidiag_doubles<ORDER>(), links = 5 * a.nplink;
+    double *vec = smem + (mats > links ? mats : links);
+    double *Ws = vec + warp * 2 * (n + 2), *Rs = Ws + (n + 2);  // the warp's bidiagonal
+    double *tmp = vec + (T / 32) * 2 * (n + 2), *bl = tmp + n, *bx = bl + n, *by = bx + n, *R = by + n;
+    double *lx = smem, *ly = lx + a.nplink, *dl = ly + a.nplink, *dxv = dl + a.nplink, *dyv = dxv + a.nplink;
+    double *M = a.M + (size_t)blockIdx.x * n * ld;
     const WArgs &wa = a.w;
     constexpr double amp_tol = 1.0001;
     constexpr int nk = 32;
-    for (int i = blockIdx.x * wpb + warp; i < wa.npfb; i += gridDim.x * wpb) {
+    const int urow = tid - n;  // 0..3: a thread on a row of U
+    double *row = tid < n ? V + tid : U + (urow < 3 ? urow : 4);
+    const bool turns = tid < n + kAdaptUrows, on_u = tid >= n;
+    // svdlib.F90:173-278; false where it does not converge (in every thread alike)
+    auto qr = [&](double anorm) -> bool {
+        for (int j = 1 + lane; j <= n; j += 32) { Ws[j] = W[j]; Rs[j] = rv1[j]; }
+        __syncwarp();
+        for (int k = n; k >= 1; k--) {
+            for (int its = 1; its <= 30; its++) {
+                bool to2000 = false;
+                int l, nm = 1;
+                for (l = k; l >= 1; l--) {
+                    nm = l - 1;
+                    if ((fabs(Rs[l]) + anorm) == anorm) { to2000 = true; break; }
+                    if ((fabs(Ws[nm]) + anorm) == anorm) break;
+                }
+                if (l < 1) return false;  // only a NaN in the bidiagonal gets here
+                double c, s, f, g, h, x, y, z;
+                if (!to2000) {
+                    c = 0.0; s = 1.0;
+                    for (int i = l; i <= k; i++) {
+                        const double r = Rs[i];
+                        f = s * r;
+                        __syncwarp();
+                        if (lane == 0) Rs[i] = c * r;
+                        if ((fabs(f) + anorm) == anorm) break;
+                        g = Ws[i];
+                        h = nr_hypot(f, g);
+                        __syncwarp();
+                        if (lane == 0) Ws[i] = h;
+                        h = 1.0 / h;
+                        c = (g * h);
+                        s = -(f * h);
+                        if (turns && on_u) {
+                            const double yy = row[(nm - 1) * ld], zz = row[(i - 1) * ld];
+                            row[(nm - 1) * ld] = (yy * c) + (zz * s);
+                            row[(i - 1) * ld] = -(yy * s) + (zz * c);
+                        }
+                    }
+                    __syncwarp();
+                }
+                z = Ws[k];
+                if (l == k) {
+                    if (z < 0.0) {
+                        __syncwarp();
+                        if (lane == 0) Ws[k] = -z;
+                        if (turns && !on_u) row[(k - 1) * ld] = -row[(k - 1) * ld];
+                    }
+                    __syncwarp();
+                    break;
+                }
+                if (its >= 30) return false;
+                x = Ws[l];
+                nm = k - 1;
+                y = Ws[nm];
+                g = Rs[nm];
+                h = Rs[k];
+                f = ((y - z) * (y + z) + (g - h) * (g + h)) / ((2.0 * h) * y);
+                g = nr_hypot(f, 1.0);
+                f = ((x - z) * (x + z) + h * ((y / (f + copysign(g, f))) - h)) / x;
+                c = 1.0; s = 1.0;
+                double xr = turns ? row[(l - 1) * ld] : 0.0;  // the row's column j, on its way to column j + 1
+                for (int j = l; j <= nm; j++) {
+                    const int i = j + 1;
+                    // entries j + 1 are read here and not written before the next j; a lane reads
+                    // them before lane 0 gets there (the warp runs the scalars in step)
+                    g = Rs[i];
+                    y = Ws[i];
+                    h = s * g;
+                    g = c * g;
+                    z = nr_hypot(f, h);
+                    __syncwarp();
+                    if (lane == 0) Rs[j] = z;
+                    c = f / z;
+                    s = h / z;
+                    const double c1 = c, s1 = s;
+                    f = (x * c) + (g * s);
+                    g = -(x * s) + (g * c);
+                    h = y * s;
+                    y = y * c;
+                    z = nr_hypot(f, h);
+                    if (lane == 0) Ws[j] = z;
+                    if (z != 0.0) {
+                        z = 1.0 / z;
+                        c = f * z;
+                        s = h * z;
+                    }
+                    f = (c * g) + (s * y);
+                    x = -(s * g) + (c * y);
+                    if (turns) {
+                        const double cr = on_u ? c : c1, sr = on_u ? s : s1;
+                        const double zr = row[(i - 1) * ld];
+                        row[(j - 1) * ld] = (xr * cr) + (zr * sr);
+                        xr = -(xr * sr) + (zr * cr);
+                    }
+                }
+                if (turns) row[(k - 1) * ld] = xr;
+                __syncwarp();
+                if (lane == 0) {
+                    Rs[l] = 0.0;
+                    Rs[k] = f;
+                    Ws[k] = x;
+                }
+                __syncwarp();
+            }
+        }
+        return true;
+    };
+    for (;;) {
+        sync();
+        if (tid == 0) sh_i = atomicAdd(a.next, 1);
+        sync();
+        const int i = sh_i;
+        if (i >= wa.npfb) return;
         const int t = wa.ntype[i];
         if (t <= 2 || t == 998) continue;
         const double xi = wa.px[i], yi = wa.py[i], si = a.sp[i];
@@ -1526,70 +1633,93 @@ __global__ void k_adapt_stencils(AdaptArgs a) {
             for (int ii = 0;; ii++) {
                 const double hh = (pass ? hs_i : h_i) * a.rf;
                 const int cur = pass ? c_small : c_all;
-                int cnt = cur;  // leading links within hh * ss
-                for (int b = 0; b < cur; b += 32) {
-                    const int k = b + lane;
-                    bool out = false;
-                    if (k < cur) {
-                        const int p = wa.lpt[sell_off(wa.slice_ptr, i, k)];
-                        const double rx = xi - wa.px[p], ry = yi - wa.py[p];
-                        out = !(sqrt(rx * rx + ry * ry) <= hh * kSs);
+                // leading links within hh * ss
+                sync();
+                if (tid == 0) { sh_cnt = cur; sh_bad = 0; }
+                sync();
+                for (int k = tid; k < cur; k += T) {
+                    const int p = wa.lpt[sell_off(wa.slice_ptr, i, k)];
+                    const double rx = xi - wa.px[p], ry = yi - wa.py[p];
+                    if (!(sqrt(rx * rx + ry * ry) <= hh * kSs)) {
+                        atomicMin(&sh_cnt, k);
+                        break;
                     }
-                    const unsigned m = __ballot_sync(0xffffffffu, out);
-                    if (m) { cnt = b + __ffs(m) - 1; break; }
                 }
-                assemble<ORDER>(wa, i, cnt, hh, U, ld, X, G, lane);
-                for (int e = lane; e < n * ld; e += 32) M[e] = U[e];
-                __syncwarp();
+                sync();
+                const int cnt = sh_cnt;
+                const double anorm = moment_bidiag<ORDER>(wa, i, cnt, hh, n, smem, U, V, W, rv1, M);
+                sync();
                 const double thr = res_tol / hh;
                 double hc;
-                if (svd_factor_warp<n>(U, V, W, rv1, ld, lane)) {
+                if (!qr(anorm)) {
                     hc = (2.0 * res_tol) / hh;
                 } else {
-                    for (int m = lane; m < n; m += 32) {
-                        bl[m] = (m == 2 || m == 4) ? (1.0 / hh) / hh : 0.0;
-                        bx[m] = m == 0 ? 1.0 / hh : 0.0;
-                        by[m] = m == 1 ? 1.0 / hh : 0.0;
-                    }
-                    svd_apply_warp<n>(U, V, W, tmp, bl, ld, lane);
-                    svd_apply_warp<n>(U, V, W, tmp, bx, ld, lane);
-                    svd_apply_warp<n>(U, V, W, tmp, by, ld, lane);
+                    sync();  // every row is in place (and the matrix in memory)
+                    const double v2 = (1.0 / hh) / hh, v1 = 1.0 / hh;
+                    auto solve = [&](double *b, int r0, int r1, double v) {
+                        if (tid < n) {
+                            double sum = 0.0;
+                            const double w = Ws[tid + 1];
+                            if (w != 0.0) {
+                                sum = sum + U[tid * ld + r0] * v;
+                                if (r1 >= 0) sum = sum + U[tid * ld + r1] * v;
+                                sum = sum / w;
+                            }
+                            tmp[tid] = sum;
+                        }
+                        sync();
+                        if (tid < n) {
+                            double sum = 0.0;
+#pragma unroll 4
+                            for (int jj = 0; jj < n; jj++) sum = sum + V[jj * ld + tid] * tmp[jj];
+                            b[tid] = sum;
+                        }
+                        sync();
+                    };
+                    solve(bl, 2, 4, v2);
+                    solve(bx, 0, -1, v1);
+                    solve(by, 1, -1, v1);
                     // residual of the Laplacian system, rows in parallel, sums in order
-                    for (int r = lane; r < n; r += 32) {
-                        double v = (r == 2 || r == 4) ? (-1.0 / hh) / hh : 0.0;
-                        for (int c = 0; c < n; c++) v = v + M[c * ld + r] * bl[c];
-                        R[r] = v;
+                    if (tid < n) {
+                        double v = (tid == 2 || tid == 4) ? (-1.0 / hh) / hh : 0.0;
+#pragma unroll 4
+                        for (int c = 0; c < n; c++) v = v + M[c * ld + tid] * bl[c];
+                        R[tid] = v;
                     }
-                    __syncwarp();
-                    hc = 0.0;
-                    if (lane == 0) {
-                        for (int r = 0; r < n; r++) hc = hc + R[r] * R[r];
-                        hc = (hc * hh) * hh;
-                        hc = sqrt(hc / (double)n);
+                    sync();
+                    if (tid == 0) {
+                        double q = 0.0;
+                        for (int r = 0; r < n; r++) q = q + R[r] * R[r];
+                        q = (q * hh) * hh;
+                        sh_hc = sqrt(q / (double)n);
                     }
-                    hc = __shfl_sync(0xffffffffu, hc, 0);
+                    sync();
+                    hc = sh_hc;
                     if (hc < thr) {
                         // each link's dot products with the three solutions (independent of q)
-                        for (int k = lane; k < cnt; k += 32) {
+                        for (int k = tid; k < cnt; k += T) {
                             const int p = wa.lpt[sell_off(wa.slice_ptr, i, k)];
                             const double x = -(xi - wa.px[p]), y = -(yi - wa.py[p]);
                             const double qq = sqrt(x * x + y * y) / hh;
                             const double ff1 = wab(qq, wa.h2);
                             const double xx = x / hh, yy = y / hh;
+                            double hx[ORDER + 1], hy[ORDER + 1];
+#pragma unroll
+                            for (int d = 0; d <= ORDER; d++) { hx[d] = hermite(d, xx); hy[d] = hermite(d, yy); }
                             double sl = 0.0, sx = 0.0, sy = 0.0;
+#pragma unroll
                             for (int m = 0; m < n; m++) {
                                 const int pm = p_of(m), qm = q_of(m);
-                                const double g = ((qm == 0) ? hermite(pm, xx) : (pm == 0) ? hermite(qm, yy)
-                                                                                          : hermite(pm, xx) * hermite(qm, yy)) * ff1;
+                                const double g = ((qm == 0) ? hx[pm] : (pm == 0) ? hy[qm] : hx[pm] * hy[qm]) * ff1;
                                 sl = sl + bl[m] * g;
                                 sx = sx + bx[m] * g;
                                 sy = sy + by[m] * g;
                             }
                             lx[k] = x; ly[k] = y; dl[k] = sl; dxv[k] = sx; dyv[k] = sy;
                         }
-                        __syncwarp();
+                        sync();
                         bool fail = false;
-                        for (int i1 = lane + 1; i1 <= nk + 1; i1 += 32) {
+                        for (int i1 = tid + 1; i1 <= nk + 1; i1 += T) {
                             const double q = (((double)i1 * kPi) / si) / (double)nk;
                             double hl = 0.0, hx = 0.0, hy = 0.0;
                             for (int k = 0; k < cnt; k++) {
@@ -1603,7 +1733,9 @@ __global__ void k_adapt_stencils(AdaptArgs a) {
                             hy = hy / q;
                             if (hl > amp_tol || hl < 0.0 || fabs(hx) > amp_tol || fabs(hy) > amp_tol) fail = true;
                         }
-                        if (__any_sync(0xffffffffu, fail)) hc = (2.0 * res_tol) / hh;
+                        if (fail) sh_bad = 1;
+                        sync();
+                        if (sh_bad) hc = (2.0 * res_tol) / hh;
                     }
                 }
                 if ((double)ii > a.limit) hc = (2.0 * res_tol) / hh;
@@ -1617,10 +1749,9 @@ __global__ void k_adapt_stencils(AdaptArgs a) {
                     hs_i = hh;
                     c_small = cnt;
                 }
-                __syncwarp();
             }
         }
-        if (lane == 0) {
+        if (tid == 0) {
             a.h[i] = h_i;
             a.hs[i] = hs_i;
         }
@@ -1723,22 +1854,22 @@ int launch_weights(Handle *H, WArgs &a) {
 
 template <int ORDER>
 int launch_adapt(Handle *H, AdaptArgs &a) {
-    const int per_warp = (adapt_fixed_doubles<ORDER>() + 5 * a.nplink + 1) & ~1;
-    const size_t per_warp_bytes = (size_t)per_warp * sizeof(double);
-    int optin = 0;
+    constexpr int n = nsz(ORDER), T = bidiag_threads(ORDER);
+    const size_t smem = (size_t)adapt_doubles<ORDER>(a.nplink) * sizeof(double);
+    int optin = 0, nsm = 0, per_sm = 0;
     if (int rc = smem_optin(H, &optin)) return rc;
-    int wpb = (int)((size_t)optin / per_warp_bytes);
-    if (wpb > 16) wpb = 16;
-    if (wpb < 1) return set_err(H, SUNSET_ERR_SCOPE, "neighbour lists too long for the stencil adaptation");
-    a.per_warp = per_warp;
-    const size_t smem = (size_t)wpb * per_warp_bytes;
+    if (smem + 1024 > (size_t)optin) return set_err(H, SUNSET_ERR_SCOPE, "neighbour lists too long for the stencil adaptation");
     SUNSET_CUDA(H, cudaFuncSetAttribute(k_adapt_stencils<ORDER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int nsm = 0;
     SUNSET_CUDA(H, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, H->device));
-    int nb = (a.w.npfb + wpb - 1) / wpb;
-    if (nb > nsm * 8) nb = nsm * 8;
-    k_adapt_stencils<ORDER><<<nb, wpb * 32, smem, H->stream>>>(a);
+    SUNSET_CUDA(H, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_adapt_stencils<ORDER>, T, smem));
+    const int nb = std::max(1, std::min(a.w.npfb, nsm * std::max(1, per_sm)));  // each takes one node after another
+    if (dalloc(H, &a.M, (size_t)nb * n * (n | 1)) || dalloc(H, &a.next, 1)) return SUNSET_ERR_NOMEM;
+    SUNSET_CUDA(H, cudaMemsetAsync(a.next, 0, sizeof(int), H->stream));
+    k_adapt_stencils<ORDER><<<nb, T, smem, H->stream>>>(a);
     SUNSET_CUDA(H, cudaGetLastError());
+    SUNSET_CUDA(H, cudaStreamSynchronize(H->stream));
+    dfree(H, a.M);
+    dfree(H, a.next);
     return 0;
 }
 
