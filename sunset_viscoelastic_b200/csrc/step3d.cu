@@ -61,7 +61,9 @@ enum G3 {
 
 // sign class of a field at a mirror image: 0 none, 1 like u (x mirrors), 2 like v (y
 // mirrors), 3 like c_xy (one of the two); code = vrelation - 1 (1 x, 2 y, 3 both)
+template <bool MIR = true>
 __device__ __forceinline__ double mirror_value(double x, int cls, int code) {
+    if (!MIR) return x;
     const bool flip = (cls == 1 && (code == 1 || code == 3)) || (cls == 2 && (code == 2 || code == 3)) ||
                       (cls == 3 && (code == 1 || code == 2));
     return flip ? -x : x;
@@ -149,31 +151,32 @@ __host__ __device__ constexpr FDesc desc3f(int d) {
 // Every derivative the right-hand side reads, in one pass over each node's links: the x-y
 // LABFM sums of all fields (in the reference's link order, each sum as calc_gradient /
 // calc_laplacian forms it), then the z stencils.  The layers of a node share its links, so a
-// warp's link and weight loads are one broadcast each.  The links go in pairs whose field
-// values are all loaded before either is summed, so that a warp keeps two links' gathers in
-// flight (the sums still run in link order).
-// Minimum resident blocks a SM asked of the compiler: the direct form's gather runs fastest at
-// 5 (96 registers); the forms with 16 gathered fields lose their loads in flight at that size
-// and run at 4 (128 registers).
-#ifndef SUNSET_3D_BLOCKS_DI
-#define SUNSET_3D_BLOCKS_DI 5
-#endif
+// warp's link and weight loads are one broadcast each.  The links go in batches whose field
+// values are all loaded before any is summed (the sums still run in link order): the kernel
+// waits for those loads, so what counts is how many a SM has in flight, links a batch times
+// resident warps, and that the registers hold them.
+//   direct form (10 fields): 4 links, 4 blocks a SM (128 registers).  128^2 x 128 layers at order 4
+//   2.78 -> 2.50 ms a step (2 links and 5 blocks before), 90^2 x 64 at order 6 1.26 -> 1.06; 3, 5, 6
+//   or 8 links, or 3, 5 or 6 blocks, are slower.
+//   Cholesky and log-conformation (10 to 16 fields): 2 links, 4 blocks, with the next links' indices
+//   fetched a batch ahead so that the field loads do not wait for them.  Cholesky at order 6, 90^2 x
+//   65 1.99 -> 1.81 ms; log-conformation at order 6, 96^2 x 65 3.00 -> 2.95 (4 links 2.93 and 3
+//   blocks 2.87 there, but 0.31 -> 0.36 at 50^2 x 30); the direct form loses by it (2.90).
 #ifndef SUNSET_3D_BLOCKS
 #define SUNSET_3D_BLOCKS 4
 #endif
-__host__ __device__ constexpr int derivs_min_blocks(int form) {
-    return form == SUNSET_FORM_DI ? SUNSET_3D_BLOCKS_DI : SUNSET_3D_BLOCKS;
-}
+__host__ __device__ constexpr int links_in_flight(int form) { return form == SUNSET_FORM_DI ? 4 : 2; }
 
 //
 // ST(slot, value) receives each derivative: a global array of the standalone gather, or the
 // fused stage kernel's shared memory.
 // BND: the node set has boundary nodes, whose conformation Laplacians (fields 7-12) take the
-// weights wlc and sums lsumc.
-template <int FORM, bool MD, bool FULL, bool FEN, bool BND, class ST>
+// weights wlc and sums lsumc.  MIR: the set has mirror links; without, their signs are compiled out.
+template <int FORM, bool MD, bool FULL, bool FEN, bool BND, bool MIR, class ST>
 __device__ __forceinline__ void derivs3_body(const Layer3 &L, const Fields3 &F, const ZThread &z, ST store) {
     constexpr int N = ndesc3<FORM, MD, FEN>();
-    constexpr int LB = 2;
+    constexpr int LB = links_in_flight(FORM);
+    constexpr bool AHEAD = LB == 2;  // fetch the next links' indices a batch ahead
     constexpr bool kCL = BND && MD;
     const int k = z.k, i = z.i, iz = z.iz, row = i * L.nz, h = L.ncfd / 2;
     double sx[N], sy[N], sl[N];
@@ -182,15 +185,24 @@ __device__ __forceinline__ void derivs3_body(const Layer3 &L, const Fields3 &F, 
     const long long base = L.slice_ptr[i >> 5];
     const int cs = L.cnt_small[i];
     int q = 0;
+    int ln[LB];
+    if (AHEAD) {
+#pragma unroll
+        for (int b = 0; b < LB; b++) ln[b] = __ldg(L.lidx + sell_at(base, min(b, max(cs - 1, 0)), i & 31));
+    }
     for (; q + LB <= cs; q += LB) {
         int pj[LB], code[LB];
         double wx[LB], wy[LB], wl[LB], wc[LB], v[LB][N];
 #pragma unroll
         for (int b = 0; b < LB; b++) {
-            const long long o = sell_at(base, q + b, i & 31);
-            const int l = __ldg(L.lidx + o);
+            const int l = AHEAD ? ln[b] : __ldg(L.lidx + sell_at(base, q + b, i & 31));
             pj[b] = (l & kLinkMask) * L.nz + iz;
             code[b] = (int)((unsigned)l >> 30);
+        }
+#pragma unroll
+        for (int b = 0; b < LB; b++) {
+            if (AHEAD) ln[b] = __ldg(L.lidx + sell_at(base, min(q + LB + b, cs - 1), i & 31));
+            const long long o = sell_at(base, q + b, i & 31);
             wx[b] = __ldg(L.wx + o);
             wy[b] = __ldg(L.wy + o);
             wl[b] = __ldg(L.wl + o);
@@ -205,7 +217,7 @@ __device__ __forceinline__ void derivs3_body(const Layer3 &L, const Fields3 &F, 
 #pragma unroll
             for (int d = 0; d < N; d++) {
                 const FDesc D = desc3f<FORM, MD, FULL, FEN>(d);
-                const double x = mirror_value(v[b][d], D.cls, code[b]);
+                const double x = mirror_value<MIR>(v[b][d], D.cls, code[b]);
                 if (D.gx >= 0) sx[d] = sx[d] + x * wx[b];
                 if (D.gy >= 0) sy[d] = sy[d] + x * wy[b];
                 if (D.gl >= 0) sl[d] = sl[d] + x * ((kCL && D.f >= 7) ? wc[b] : wl[b]);
@@ -221,7 +233,7 @@ __device__ __forceinline__ void derivs3_body(const Layer3 &L, const Fields3 &F, 
 #pragma unroll
         for (int d = 0; d < N; d++) {
             const FDesc D = desc3f<FORM, MD, FULL, FEN>(d);
-            const double x = mirror_value(F.p[D.f][pj], D.cls, code);
+            const double x = mirror_value<MIR>(F.p[D.f][pj], D.cls, code);
             if (D.gx >= 0) sx[d] = sx[d] + x * wx;
             if (D.gy >= 0) sy[d] = sy[d] + x * wy;
             if (D.gl >= 0) sl[d] = sl[d] + x * ((kCL && D.f >= 7) ? wc : wl);
@@ -991,15 +1003,15 @@ __device__ __forceinline__ void block_emax3(unsigned long long eb, DevScalars *s
 // One stage fused: the derivatives of node-layer k (derivs3_body) go to this block's shared
 // memory, compact slots of 128 doubles (one per thread), and the pointwise right-hand side
 // and RK update (point3_body) read them there, so no derivative array crosses HBM.
-template <int FORM, bool MD, bool FULL, bool FEN, bool BND>
-__global__ void __launch_bounds__(128, derivs_min_blocks(FORM)) k3_stage(Layer3 L, Fields3 F, Point3 P) {
+template <int FORM, bool MD, bool FULL, bool FEN, bool BND, bool MIR>
+__global__ void __launch_bounds__(128, SUNSET_3D_BLOCKS) k3_stage(Layer3 L, Fields3 F, Point3 P) {
     constexpr int NS = ngslots<FORM, MD, FULL, FEN>();
     __shared__ double sg[NS * 128];
     ZThread z;
     const bool live = zthread(L, z);
     unsigned long long eb = 0;
     if (live) {
-        derivs3_body<FORM, MD, FULL, FEN, BND>(L, F, z, [&](int slot, double v) {
+        derivs3_body<FORM, MD, FULL, FEN, BND, MIR>(L, F, z, [&](int slot, double v) {
             const int c = kGTable<FORM, MD, FULL, FEN>.idx[slot];
             if (c >= 0) sg[c * 128 + threadIdx.x] = v;
         });
@@ -1399,9 +1411,11 @@ int stage3_launch(Handle *H, int b, int stage) {
         F.p[19] = H->tmp3;
     }
     if (H->nb > 0)
-        k3_stage<FORM, MD, FULL, FEN, true><<<zblocks(H), 128, 0, H->stream>>>(layer3(H), F, point3(H, b, stage));
+        k3_stage<FORM, MD, FULL, FEN, true, true><<<zblocks(H), 128, 0, H->stream>>>(layer3(H), F, point3(H, b, stage));
+    else if (H->has_mirrors)
+        k3_stage<FORM, MD, FULL, FEN, false, true><<<zblocks(H), 128, 0, H->stream>>>(layer3(H), F, point3(H, b, stage));
     else
-        k3_stage<FORM, MD, FULL, FEN, false><<<zblocks(H), 128, 0, H->stream>>>(layer3(H), F, point3(H, b, stage));
+        k3_stage<FORM, MD, FULL, FEN, false, false><<<zblocks(H), 128, 0, H->stream>>>(layer3(H), F, point3(H, b, stage));
     SUNSET_CUDA(H, cudaGetLastError());
     return 0;
 }
