@@ -391,7 +391,7 @@ __device__ __forceinline__ long long sell_off(const long long *slice_ptr, int i,
 // A node whose rotations do not fit its record stops before the sweep that would not fit, and
 // the last two kernels run again until every node is done.
 //
-// 1,048,576 nodes at order 8: 1943 -> 515 ms (262,144: 99 + 7 + 18 ms in the three kernels).
+// 262,144 nodes at order 8: 83 + 7 + 18 ms in the three kernels; 1,048,576: 1943 -> 450 ms.
 // ---------------------------------------------------------------------------------------
 constexpr int kUrows = 10;  // rows of U the solves read: 0, 1, 2, 4 and up to six of the filter's
 
@@ -431,15 +431,19 @@ struct SvdBatch {
 };
 
 __host__ __device__ constexpr int bidiag_threads(int order) { return (nsz(order) + 31) / 32 * 32; }
-constexpr int kAsmLinks = 32;  // links whose monomials are staged at once
-// Doubles of shared memory of k_moment_bidiag: U, V and three vectors; while the moment
-// matrix is assembled, U's and V's place holds the chunk's powers, Hermite polynomials and
-// monomials.
+constexpr int kAsmLinks = 16;  // links whose monomials are staged at once
+// Doubles of shared memory of moment_bidiag: the matrix (while the moment matrix is assembled, its
+// place holds the links' powers, Hermite polynomials and monomials), a staged row, and the
+// bidiagonal.
 template <int ORDER>
-__host__ __device__ constexpr int bidiag_doubles() {
-    constexpr int n = nsz(ORDER), mats = 2 * n * (n | 1), stage = kAsmLinks * (4 * (ORDER + 1) + 1 + n);
-    return (mats > stage ? mats : stage) + 2 * (n + 2);
+__host__ __device__ constexpr int bidiag_matrix() {
+    constexpr int n = nsz(ORDER), mat = n * (n | 1), stage = kAsmLinks * (4 * (ORDER + 1) + 1 + n) + 2;
+    return mat > stage ? mat : stage;
 }
+template <int ORDER>
+__host__ __device__ constexpr int bidiag_doubles() { return bidiag_matrix<ORDER>() + (nsz(ORDER) + 2) + 2 * (nsz(ORDER) + 2); }
+// Blocks a SM that shared memory leaves room for; the registers are held to them.
+__host__ __device__ constexpr int bidiag_blocks(int order) { return order <= 6 ? 24 : order == 8 ? 12 : 6; }
 
 // Whether the filter's moment matrix is the derivative one (labf.F90:258-303).
 __device__ __forceinline__ bool same_matrix(const WArgs &a, int i, int t) {
@@ -458,16 +462,24 @@ __global__ void k_weight_items(WArgs a, int *item0, int *item1, int *count) {
 }
 
 // A block's moment matrix over links [0, cnt) with length hh (labf.F90:88-148 or 258-303; only the
-// first `keep` unknowns, the identity beyond) and svdlib.F90:37-171: on return U and V are the
-// accumulated transformations (column-major, leading dimension n | 1) and W, rv1 (1-based) the
-// bidiagonal, all in shared memory (bidiag_doubles of it at smem, U first); returns anorm.  M, if
-// not null, gets the matrix.  Bound: the FP64 sums in the reference's serial order (a
-// column's dot product is one chain), six blocks of two warps a SM at order 8.
-template <int ORDER>
-__device__ double moment_bidiag(const WArgs &a, int i0, int cnt, double hh, int keep, double *smem, double *U, double *V,
-                                double *W, double *rv1, double *M) {
+// first `keep` unknowns, the identity beyond) and svdlib.F90:37-171.  One n x n matrix of
+// shared memory (column-major, leading dimension n | 1, at smem) serves in turn for the bidiagonalisation, the
+// accumulation of U, of which take_u(U) copies what it wants, and that of V, which it holds on
+// return with the bidiagonal W, rv1 (1-based); returns anorm.  M (n x n doubles in memory) gets the
+// moment matrix, column by column, and rows (as large) the bidiagonalised one, row by row.
+//
+// Bound: latency.  A dependent FP64 operation takes some 25 cycles here, and the sums are single
+// chains in the reference's order, so what counts is how many nodes a SM has under way: with both
+// matrices in shared memory and the moment matrix's columns in registers they were six at order 8
+// (162 registers), now twelve (262,144 nodes 99 -> 83 ms; order 6, twenty-four blocks, 21 -> 17).
+// Holding a thread's column in registers across a step's two loops, with 16-byte loads of the
+// Householder vector, saved instructions and shared-memory traffic but no time (103 ms).
+template <int ORDER, class TAKEU>
+__device__ __forceinline__ double moment_bidiag(const WArgs &a, int i0, int cnt, double hh, int keep, double *smem, double *W,
+                                                double *rv1, double *M, double *rows, TAKEU take_u) {
     constexpr int n = nsz(ORDER), ld = n | 1, T = bidiag_threads(ORDER);
     const int tid = threadIdx.x;
+    double *U = smem, *V = smem, *pv = smem + bidiag_matrix<ORDER>();
     auto sync = [] {
         if constexpr (T == 32) __syncwarp();
         else __syncthreads();
@@ -478,62 +490,63 @@ __device__ double moment_bidiag(const WArgs &a, int i0, int cnt, double hh, int 
         const int m = tid < n ? tid : 0;
         const int pm = p_of(m), qm = q_of(m);
         const double den = fact(pm) * fact(qm), inv = 1.0 / den;
-        double acc[n];
-#pragma unroll
-        for (int r = 0; r < n; r++) acc[r] = 0.0;
-        constexpr int P = ORDER + 1;
+        constexpr int P = ORDER + 1, RB = n <= 14 ? n : n <= 44 ? (n + 1) / 2 : 22;  // rows a pass over the links
         double *xp = smem, *yp = xp + kAsmLinks * P, *hx = yp + kAsmLinks * P, *hy = hx + kAsmLinks * P;
         double *ker = hy + kAsmLinks * P, *X = ker + kAsmLinks;
         const double xi = a.px[i0], yi = a.py[i0];
-        for (int k0 = 0; k0 < cnt; k0 += kAsmLinks) {
-            const int nk = min(kAsmLinks, cnt - k0);
-            sync();
-            if (tid < nk) {
-                const int p = a.lpt[sell_off(a.slice_ptr, i0, k0 + tid)];
-                const double x = -(xi - a.px[p]), y = -(yi - a.py[p]);
-                const double rad = sqrt(x * x + y * y) / hh;
-                ker[tid] = wab(rad, a.h2);
-                const double xx = x / hh, yy = y / hh;
-                double px = xx, py = yy;
-                xp[tid] = yp[tid] = 1.0;
+        for (int r0 = 0; r0 < n; r0 += RB) {
+            double acc[RB];
 #pragma unroll
-                for (int d = 1; d <= ORDER; d++) {
-                    xp[d * kAsmLinks + tid] = px;
-                    yp[d * kAsmLinks + tid] = py;
-                    px = px * xx;
-                    py = py * yy;
+            for (int r = 0; r < RB; r++) acc[r] = 0.0;
+            for (int k0 = 0; k0 < cnt; k0 += kAsmLinks) {
+                const int nk = min(kAsmLinks, cnt - k0);
+                sync();
+                // a thread a link and coordinate
+                const int kl = tid & (kAsmLinks - 1), side = tid / kAsmLinks;
+                if (side < 2 && kl < nk) {
+                    const int p = a.lpt[sell_off(a.slice_ptr, i0, k0 + kl)];
+                    const double x = -(xi - a.px[p]), y = -(yi - a.py[p]);
+                    if (side == 0) ker[kl] = wab(sqrt(x * x + y * y) / hh, a.h2);
+                    const double z = (side ? y : x) / hh;
+                    double *zp = side ? yp : xp, *hz = side ? hy : hx;
+                    double pz = z;
+                    zp[kl] = 1.0;
+#pragma unroll
+                    for (int d = 1; d <= ORDER; d++) {
+                        zp[d * kAsmLinks + kl] = pz;
+                        pz = pz * z;
+                    }
+#pragma unroll
+                    for (int d = 0; d <= ORDER; d++) hz[d * kAsmLinks + kl] = hermite(d, z);
                 }
+                sync();
+                if (tid < n)
+                    for (int k = 0; k < nk; k++) {
+                        const double xv = xp[pm * kAsmLinks + k], yv = yp[qm * kAsmLinks + k];
+                        double v;
+                        if (den == 1.0) v = pm == 0 ? yv : qm == 0 ? xv : xv * yv;
+                        else v = qm == 0 ? inv * xv : pm == 0 ? inv * yv : (inv * xv) * yv;
+                        X[k * n + tid] = v;
+                    }
+                sync();
+                for (int k = 0; k < nk; k++) {
+                    const double hxv = hx[pm * kAsmLinks + k], hyv = hy[qm * kAsmLinks + k];
+                    const double g = (qm == 0 ? hxv : pm == 0 ? hyv : hxv * hyv) * ker[k];
 #pragma unroll
-                for (int d = 0; d <= ORDER; d++) {
-                    hx[d * kAsmLinks + tid] = hermite(d, xx);
-                    hy[d * kAsmLinks + tid] = hermite(d, yy);
+                    for (int r = 0; r < RB; r++)  // (a last pass's rows beyond n are not kept)
+                        acc[r] = acc[r] + X[k * n + r0 + r] * g;
                 }
             }
-            sync();
-            if (tid < n)
-                for (int k = 0; k < nk; k++) {
-                    const double xv = xp[pm * kAsmLinks + k], yv = yp[qm * kAsmLinks + k];
-                    double v;
-                    if (den == 1.0) v = pm == 0 ? yv : qm == 0 ? xv : xv * yv;
-                    else v = qm == 0 ? inv * xv : pm == 0 ? inv * yv : (inv * xv) * yv;
-                    X[k * n + tid] = v;
-                }
-            sync();
-            for (int k = 0; k < nk; k++) {
-                const double hxv = hx[pm * kAsmLinks + k], hyv = hy[qm * kAsmLinks + k];
-                const double g = (qm == 0 ? hxv : pm == 0 ? hyv : hxv * hyv) * ker[k];
+            if (tid < n) {
 #pragma unroll
-                for (int r = 0; r < n; r++) acc[r] = acc[r] + X[k * n + r] * g;
+                for (int r = 0; r < RB; r++)
+                    if (r0 + r < n) M[tid * n + r0 + r] = acc[r];
             }
         }
         sync();
-        if (tid < n) {
-#pragma unroll
-            for (int r = 0; r < n; r++) U[tid * ld + r] = (tid >= keep || r >= keep) ? (r == tid ? 1.0 : 0.0) : acc[r];
-            if (M) {
-#pragma unroll
-                for (int r = 0; r < n; r++) M[tid * ld + r] = acc[r];
-            }
+        for (int e = tid; e < n * n; e += T) {
+            const int c = e / n, r = e - c * n;
+            U[c * ld + r] = (c >= keep || r >= keep) ? (r == c ? 1.0 : 0.0) : M[e];
         }
         sync();
     }
@@ -606,29 +619,11 @@ __device__ double moment_bidiag(const WArgs &a, int i0, int cnt, double hh, int 
         const double tn = fabs(wi) + fabs(ri);
         anorm = (tn > anorm) ? tn : anorm;
     }
-    // right-hand transformations, svdlib.F90:115-141
-    g = 0.0;
-    for (int i = n; i >= 1; i--) {
-        if (i < n) {
-            if (g != 0.0) {
-                if (me >= l && me <= n) VM(me, i) = (UM(i, me) / UM(i, l)) / g;
-                sync();
-                if (me >= l && me <= n) {
-                    double sj = 0.0;
-#pragma unroll 4
-                    for (int k = l; k <= n; k++) sj = sj + UM(i, k) * VM(k, me);
-#pragma unroll 4
-                    for (int k = l; k <= n; k++) VM(k, me) = VM(k, me) + sj * VM(k, i);
-                }
-                sync();
-            }
-            if (me >= l && me <= n) { VM(i, me) = 0.0; VM(me, i) = 0.0; }
-        }
-        if (tid == 0) VM(i, i) = 1.0;
-        sync();
-        g = rv1[i];
-        l = i;
+    for (int e = tid; e < n * n; e += T) {
+        const int r = e / n, k = e - r * n;
+        rows[e] = U[k * ld + r];
     }
+    sync();
     // left-hand transformations, svdlib.F90:143-171
     for (int i = n; i >= 1; i--) {
         l = i + 1;
@@ -654,19 +649,50 @@ __device__ double moment_bidiag(const WArgs &a, int i0, int cnt, double hh, int 
         }
         sync();
     }
+    take_u(U);
+    sync();
+    // right-hand transformations, svdlib.F90:115-141, on the rows of the bidiagonalised matrix, each
+    // fetched an i ahead
+    double next = n > 1 && me <= n ? rows[(n - 2) * n + tid] : 0.0;
+    g = 0.0;
+    for (int i = n; i >= 1; i--) {
+        if (i < n) {
+            const double u = next;
+            if (i > 1 && me <= n) next = rows[(i - 2) * n + tid];
+            if (g != 0.0) {
+                if (me <= n) pv[me] = u;
+                sync();
+                if (me >= l && me <= n) VM(me, i) = (u / pv[l]) / g;
+                sync();
+                if (me >= l && me <= n) {
+                    double sj = 0.0;
+#pragma unroll 4
+                    for (int k = l; k <= n; k++) sj = sj + pv[k] * VM(k, me);
+#pragma unroll 4
+                    for (int k = l; k <= n; k++) VM(k, me) = VM(k, me) + sj * VM(k, i);
+                }
+                sync();
+            }
+            if (me >= l && me <= n) { VM(i, me) = 0.0; VM(me, i) = 0.0; }
+        }
+        if (tid == 0) VM(i, i) = 1.0;
+        sync();
+        g = rv1[i];
+        l = i;
+    }
     return anorm;
 #undef UM
 #undef VM
 }
 
-// One item a block: its matrix and the batch's arrays.
+// One item a block: its matrix and the batch's arrays.  The item's place for V holds the moment
+// matrix before, and its record the rows.
 template <int ORDER>
-__global__ void __launch_bounds__(bidiag_threads(ORDER)) k_moment_bidiag(WArgs a, SvdBatch B) {
+__global__ void __launch_bounds__(bidiag_threads(ORDER), bidiag_blocks(ORDER)) k_moment_bidiag(WArgs a, SvdBatch B) {
     constexpr int n = nsz(ORDER), ld = n | 1, T = bidiag_threads(ORDER);
     extern __shared__ double smem[];
     const int it = blockIdx.x, tid = threadIdx.x, me = tid + 1;
     const int i0 = B.item[it], t = a.ntype[i0];
-    double *U = smem, *V = U + n * ld;
     double *rv1 = smem + bidiag_doubles<ORDER>() - 2 * (n + 2), *W = rv1 + (n + 2);
     // labf.F90:125-148, 305-323: next to walls only the first unknowns are kept
     int keep = n;
@@ -677,18 +703,20 @@ __global__ void __launch_bounds__(bidiag_threads(ORDER)) k_moment_bidiag(WArgs a
         if (a.forder >= 7 && (t == 998 || t < 0)) keep = min(keep, 27);
         if (a.forder >= 5 && t == -1) keep = min(keep, 14);
     }
-    const double anorm = moment_bidiag<ORDER>(a, i0, B.pass ? a.cnt[i0] : a.cnt_small[i0], B.pass ? a.h[i0] : a.hs[i0], keep,
-                                              smem, U, V, W, rv1, nullptr);
-    // the rows of U that the solves read, V, and the bidiagonal
-    const int fo = filter_order(a.forder, t);
-    for (int e = tid; e < kUrows * n; e += T) {
-        const int r = e / n, c = e % n;
-        double dummy;
-        int row = r < 3 ? r : 4;
-        if (r >= 4) row = hyp_entry(fo, r - 4, &dummy);
-        B.U[(size_t)it * kUrows * n + e] = row >= 0 && row < n ? U[c * ld + row] : 0.0;
-    }
-    for (int e = tid; e < n * n; e += T) B.V[(size_t)it * n * n + e] = V[(e / n) * ld + e % n];
+    double *V = B.V + (size_t)it * n * n;
+    const double anorm = moment_bidiag<ORDER>(
+        a, i0, B.pass ? a.cnt[i0] : a.cnt_small[i0], B.pass ? a.h[i0] : a.hs[i0], keep, smem, W, rv1, V,
+        reinterpret_cast<double *>(B.rec + (size_t)it * B.cap), [&](const double *U) {  // the rows that the solves read
+            const int fo = filter_order(a.forder, t);
+            for (int e = tid; e < kUrows * n; e += T) {
+                const int r = e / n, c = e % n;
+                double dummy;
+                int row = r < 3 ? r : 4;
+                if (r >= 4) row = hyp_entry(fo, r - 4, &dummy);
+                B.U[(size_t)it * kUrows * n + e] = row >= 0 && row < n ? U[c * ld + row] : 0.0;
+            }
+        });
+    for (int e = tid; e < n * n; e += T) V[e] = smem[(e / n) * ld + e % n];
     if (me <= n) {
         B.W[(size_t)me * B.batch + it] = W[me];
         B.rv1[(size_t)me * B.batch + it] = rv1[me];
@@ -1462,7 +1490,7 @@ struct AdaptArgs {
     WArgs w;
     double *h, *hs;
     const double *sp;
-    double *M;  // a moment matrix a block
+    double *M;  // a block's moment matrix and its rows
     int *next;  // the next node to take
     int nplink;
     double rf, limit, res_tol[2];
@@ -1471,15 +1499,18 @@ struct AdaptArgs {
 // Rows of U that the three solves read: 0, 1, 2 and 4.
 constexpr int kAdaptUrows = 4;
 template <int ORDER>
-__host__ __device__ constexpr int adapt_vectors() {  // the warps' bidiagonals, tmp, bl, bx, by, residual
-    return (bidiag_threads(ORDER) / 32) * 2 * (nsz(ORDER) + 2) + 5 * nsz(ORDER) + 8;
+__host__ __device__ constexpr int adapt_vectors() {  // the warps' bidiagonals, tmp, bl, bx, by, residual, U's rows
+    return (bidiag_threads(ORDER) / 32) * 2 * (nsz(ORDER) + 2) + (5 + kAdaptUrows) * nsz(ORDER) + 8;
 }
-// The links' coordinates and dot products take the place of U and V, which are used up by then.
+// The links' coordinates and dot products take the place of V, which is used up by then.
 template <int ORDER>
 __host__ __device__ inline int adapt_doubles(int nplink) {
     const int mats = bidiag_doubles<ORDER>(), links = 5 * nplink;
     return (mats > links ? mats : links) + adapt_vectors<ORDER>();
 }
+
+// Blocks a SM that shared memory leaves room for; the registers are held to them.
+__host__ __device__ constexpr int adapt_blocks(int order) { return order <= 6 ? 16 : order == 8 ? 9 : 5; }
 
 // One node a block at a time.  Every length tried takes a factorisation: the block function
 // above, then the QR iteration, whose scalars every warp carries along by itself (its own copy
@@ -1487,7 +1518,7 @@ __host__ __device__ inline int adapt_doubles(int nplink) {
 // solves read.  One warp a node with all of U, V and the matrix in shared memory held four
 // nodes a SM and took 1.5 ms a factorisation at order 8.
 template <int ORDER>
-__global__ void __launch_bounds__(bidiag_threads(ORDER)) k_adapt_stencils(AdaptArgs a) {
+__global__ void __launch_bounds__(bidiag_threads(ORDER), adapt_blocks(ORDER)) k_adapt_stencils(AdaptArgs a) {
     constexpr int n = nsz(ORDER), ld = n | 1, T = bidiag_threads(ORDER);
     static_assert(n + kAdaptUrows <= T, "a thread a row");
     extern __shared__ double smem[];
@@ -1498,19 +1529,19 @@ __global__ void __launch_bounds__(bidiag_threads(ORDER)) k_adapt_stencils(AdaptA
         if constexpr (T == 32) __syncwarp();
         else __syncthreads();
     };
-    double *U = smem, *V = U + n * ld;
+    double *V = smem;
     double *rv1 = smem + bidiag_doubles<ORDER>() - 2 * (n + 2), *W = rv1 + (n + 2);
     const int mats = bidiag_doubles<ORDER>(), links = 5 * a.nplink;
     double *vec = smem + (mats > links ? mats : links);
     double *Ws = vec + warp * 2 * (n + 2), *Rs = Ws + (n + 2);  // the warp's bidiagonal
-    double *tmp = vec + (T / 32) * 2 * (n + 2), *bl = tmp + n, *bx = bl + n, *by = bx + n, *R = by + n;
+    double *tmp = vec + (T / 32) * 2 * (n + 2), *bl = tmp + n, *bx = bl + n, *by = bx + n, *R = by + n, *Ur = R + n;
     double *lx = smem, *ly = lx + a.nplink, *dl = ly + a.nplink, *dxv = dl + a.nplink, *dyv = dxv + a.nplink;
-    double *M = a.M + (size_t)blockIdx.x * n * ld;
+    double *M = a.M + (size_t)blockIdx.x * 2 * n * n, *rows = M + n * n;
     const WArgs &wa = a.w;
     constexpr double amp_tol = 1.0001;
     constexpr int nk = 32;
-    const int urow = tid - n;  // 0..3: a thread on a row of U
-    double *row = tid < n ? V + tid : U + (urow < 3 ? urow : 4);
+    double *row = tid < n ? V + tid : Ur + (tid - n) * n;  // a row of V, or one of U's (0, 1, 2 and 4)
+    const int step = tid < n ? ld : 1;
     const bool turns = tid < n + kAdaptUrows, on_u = tid >= n;
     // svdlib.F90:173-278; false where it does not converge (in every thread alike)
     auto qr = [&](double anorm) -> bool {
@@ -1543,9 +1574,9 @@ __global__ void __launch_bounds__(bidiag_threads(ORDER)) k_adapt_stencils(AdaptA
                         c = (g * h);
                         s = -(f * h);
                         if (turns && on_u) {
-                            const double yy = row[(nm - 1) * ld], zz = row[(i - 1) * ld];
-                            row[(nm - 1) * ld] = (yy * c) + (zz * s);
-                            row[(i - 1) * ld] = -(yy * s) + (zz * c);
+                            const double yy = row[(nm - 1) * step], zz = row[(i - 1) * step];
+                            row[(nm - 1) * step] = (yy * c) + (zz * s);
+                            row[(i - 1) * step] = -(yy * s) + (zz * c);
                         }
                     }
                     __syncwarp();
@@ -1555,7 +1586,7 @@ __global__ void __launch_bounds__(bidiag_threads(ORDER)) k_adapt_stencils(AdaptA
                     if (z < 0.0) {
                         __syncwarp();
                         if (lane == 0) Ws[k] = -z;
-                        if (turns && !on_u) row[(k - 1) * ld] = -row[(k - 1) * ld];
+                        if (turns && !on_u) row[(k - 1) * step] = -row[(k - 1) * step];
                     }
                     __syncwarp();
                     break;
@@ -1570,7 +1601,7 @@ __global__ void __launch_bounds__(bidiag_threads(ORDER)) k_adapt_stencils(AdaptA
                 g = nr_hypot(f, 1.0);
                 f = ((x - z) * (x + z) + h * ((y / (f + copysign(g, f))) - h)) / x;
                 c = 1.0; s = 1.0;
-                double xr = turns ? row[(l - 1) * ld] : 0.0;  // the row's column j, on its way to column j + 1
+                double xr = turns ? row[(l - 1) * step] : 0.0;  // the row's column j, on its way to column j + 1
                 for (int j = l; j <= nm; j++) {
                     const int i = j + 1;
                     // entries j + 1 are read here and not written before the next j; a lane reads
@@ -1600,12 +1631,12 @@ __global__ void __launch_bounds__(bidiag_threads(ORDER)) k_adapt_stencils(AdaptA
                     x = -(s * g) + (c * y);
                     if (turns) {
                         const double cr = on_u ? c : c1, sr = on_u ? s : s1;
-                        const double zr = row[(i - 1) * ld];
-                        row[(j - 1) * ld] = (xr * cr) + (zr * sr);
+                        const double zr = row[(i - 1) * step];
+                        row[(j - 1) * step] = (xr * cr) + (zr * sr);
                         xr = -(xr * sr) + (zr * cr);
                     }
                 }
-                if (turns) row[(k - 1) * ld] = xr;
+                if (turns) row[(k - 1) * step] = xr;
                 __syncwarp();
                 if (lane == 0) {
                     Rs[l] = 0.0;
@@ -1647,7 +1678,12 @@ __global__ void __launch_bounds__(bidiag_threads(ORDER)) k_adapt_stencils(AdaptA
                 }
                 sync();
                 const int cnt = sh_cnt;
-                const double anorm = moment_bidiag<ORDER>(wa, i, cnt, hh, n, smem, U, V, W, rv1, M);
+                const double anorm = moment_bidiag<ORDER>(wa, i, cnt, hh, n, smem, W, rv1, M, rows, [&](const double *U) {
+                    for (int e = tid; e < kAdaptUrows * n; e += T) {
+                        const int r = e / n;
+                        Ur[e] = U[(e - r * n) * ld + (r < 3 ? r : 4)];
+                    }
+                });
                 sync();
                 const double thr = res_tol / hh;
                 double hc;
@@ -1661,8 +1697,8 @@ __global__ void __launch_bounds__(bidiag_threads(ORDER)) k_adapt_stencils(AdaptA
                             double sum = 0.0;
                             const double w = Ws[tid + 1];
                             if (w != 0.0) {
-                                sum = sum + U[tid * ld + r0] * v;
-                                if (r1 >= 0) sum = sum + U[tid * ld + r1] * v;
+                                sum = sum + Ur[r0 * n + tid] * v;
+                                if (r1 >= 0) sum = sum + Ur[r1 * n + tid] * v;
                                 sum = sum / w;
                             }
                             tmp[tid] = sum;
@@ -1676,14 +1712,14 @@ __global__ void __launch_bounds__(bidiag_threads(ORDER)) k_adapt_stencils(AdaptA
                         }
                         sync();
                     };
-                    solve(bl, 2, 4, v2);
+                    solve(bl, 2, 3, v2);  // rows 2 and 4 of U
                     solve(bx, 0, -1, v1);
                     solve(by, 1, -1, v1);
                     // residual of the Laplacian system, rows in parallel, sums in order
                     if (tid < n) {
                         double v = (tid == 2 || tid == 4) ? (-1.0 / hh) / hh : 0.0;
 #pragma unroll 4
-                        for (int c = 0; c < n; c++) v = v + M[c * ld + tid] * bl[c];
+                        for (int c = 0; c < n; c++) v = v + M[c * n + tid] * bl[c];
                         R[tid] = v;
                     }
                     sync();
@@ -1863,7 +1899,7 @@ int launch_adapt(Handle *H, AdaptArgs &a) {
     SUNSET_CUDA(H, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, H->device));
     SUNSET_CUDA(H, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_adapt_stencils<ORDER>, T, smem));
     const int nb = std::max(1, std::min(a.w.npfb, nsm * std::max(1, per_sm)));  // each takes one node after another
-    if (dalloc(H, &a.M, (size_t)nb * n * (n | 1)) || dalloc(H, &a.next, 1)) return SUNSET_ERR_NOMEM;
+    if (dalloc(H, &a.M, (size_t)nb * 2 * n * n) || dalloc(H, &a.next, 1)) return SUNSET_ERR_NOMEM;
     SUNSET_CUDA(H, cudaMemsetAsync(a.next, 0, sizeof(int), H->stream));
     k_adapt_stencils<ORDER><<<nb, T, smem, H->stream>>>(a);
     SUNSET_CUDA(H, cudaGetLastError());
