@@ -583,27 +583,12 @@ int sunset_calc_gradient(SunsetHandle *sh, const double *phi, double *grad, int 
     if (int rc = op_common(sh, &H)) return rc;
     if (!phi || !grad) return set_err(H, SUNSET_ERR_ARG, "null array");
     const int n = H->npfb;
-    double *p = H->tmpd, *gx = H->tmpd + n, *gy = H->tmpd + 2 * (size_t)n;
+    double *p = H->tmpd, *g = H->tmpd + n;
     if (int rc = to_internal(H, phi, flags, p)) return rc;
-    if (int rc = op_gradient(H, p, gx, gy)) return rc;
-    std::vector<double> hx(n), hy(n);
-    double *ref = H->tmpd + 3 * (size_t)n;
-    for (int c = 0; c < 2; c++) {
-        const double *src = c == 0 ? gx : gy;
-        std::vector<double> &dst = c == 0 ? hx : hy;
-        if (int rc = to_reference(H, src, SUNSET_PTR_DEVICE, ref)) return rc;
-        SUNSET_CUDA(H, cudaMemcpyAsync(dst.data(), ref, n * sizeof(double), cudaMemcpyDeviceToHost, H->stream));
-        SUNSET_CUDA(H, cudaStreamSynchronize(H->stream));
-    }
-    if (flags == SUNSET_PTR_DEVICE) {
-        std::vector<double> inter(2 * (size_t)n);
-        for (int r = 0; r < n; r++) { inter[2 * r] = hx[r]; inter[2 * r + 1] = hy[r]; }
-        SUNSET_CUDA(H, cudaMemcpyAsync(grad, inter.data(), inter.size() * sizeof(double), cudaMemcpyHostToDevice,
-                                       H->stream));
-        SUNSET_CUDA(H, cudaStreamSynchronize(H->stream));
-    } else {
-        for (int r = 0; r < n; r++) { grad[2 * r] = hx[r]; grad[2 * r + 1] = hy[r]; }
-    }
+    if (int rc = op_gradient_ref(H, p, g)) return rc;
+    SUNSET_CUDA(H, cudaMemcpyAsync(grad, g, 2 * (size_t)n * sizeof(double),
+                                   flags == SUNSET_PTR_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, H->stream));
+    SUNSET_CUDA(H, cudaStreamSynchronize(H->stream));
     return 0;
 }
 

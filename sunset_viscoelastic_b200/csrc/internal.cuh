@@ -388,6 +388,7 @@ int step_run(Handle *H, double dt, int nsteps, int mode);
 int rhs_only(Handle *H);
 int set_tstep_device(Handle *H);
 int op_gradient(Handle *H, const double *phi, double *gx, double *gy);
+int op_gradient_ref(Handle *H, const double *phi, double *grad);  // reference order, node-major
 int op_laplacian(Handle *H, const double *phi, double *lap);
 int op_filter(Handle *H, const double *phi, double *out, int term_only);
 int reduce_ke_mass(Handle *H, double *ke, double *mass);

@@ -1536,7 +1536,11 @@ __global__ void k_tstep_fold(DevScalars *sc, StepConsts cK) {
 // ---------------------------------------------------------------------------------------
 // Single operators of the C-ABI (derivatives.F90), on a field in internal order.
 // ---------------------------------------------------------------------------------------
-__global__ void k_op_grad_lap(StageArgs A, const double *phi, double *gx, double *gy, double *lap) {
+// GRAD: the gradient, node-major in the reference's order (perm: internal -> reference node), so
+// that it leaves the device in one piece; otherwise gx, gy or lap where they are not null, in
+// internal order.
+template <bool GRAD>
+__global__ void k_op_grad_lap(StageArgs A, const double *phi, double *gx, double *gy, double *lap, const int *perm, double *grad) {
     const StepConsts &cK = A.K;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if ((i >> 5) >= cK.nslices) return;
@@ -1547,12 +1551,20 @@ __global__ void k_op_grad_lap(StageArgs A, const double *phi, double *gx, double
         const long long o = sell_at(base, k, i & 31);
         const int j = __ldg(A.lidx + o) & kLinkMask;
         const double pj = phi[j];
-        sx = sx + pj * __ldg(A.wx + o);
-        sy = sy + pj * __ldg(A.wy + o);
-        sl = sl + pj * __ldg(A.wl + o);
+        if (GRAD || gx) {
+            sx = sx + pj * __ldg(A.wx + o);
+            sy = sy + pj * __ldg(A.wy + o);
+        }
+        if (!GRAD && lap) sl = sl + pj * __ldg(A.wl + o);
     }
     if (i >= cK.npfb) return;
     const double p = phi[i];
+    if constexpr (GRAD) {
+        double *g = grad + 2 * (size_t)perm[i];
+        g[0] = sx - p * A.gsx[i];
+        g[1] = sy - p * A.gsy[i];
+        return;
+    }
     if (gx) gx[i] = sx - p * A.gsx[i];
     if (gy) gy[i] = sy - p * A.gsy[i];
     if (lap) lap[i] = sl - p * A.lsum[i];
@@ -2108,7 +2120,18 @@ int op_gradient(Handle *H, const double *phi, double *gx, double *gy) {
     if (rc) return rc;
     StageArgs A = make_args(H, 0, 5);
     const int TB = 128, nblk = (H->nslices * kSlice + TB - 1) / TB;
-    k_op_grad_lap<<<nblk, TB, 0, H->stream>>>(A, phi, gx, gy, nullptr);
+    k_op_grad_lap<false><<<nblk, TB, 0, H->stream>>>(A, phi, gx, gy, nullptr, nullptr, nullptr);
+    SUNSET_CUDA(H, cudaGetLastError());
+    return 0;
+}
+
+// The gradient in the reference's order, node-major (2 npfb).
+int op_gradient_ref(Handle *H, const double *phi, double *grad) {
+    int rc = upload_consts(H);
+    if (rc) return rc;
+    StageArgs A = make_args(H, 0, 5);
+    const int TB = 128, nblk = (H->nslices * kSlice + TB - 1) / TB;
+    k_op_grad_lap<true><<<nblk, TB, 0, H->stream>>>(A, phi, nullptr, nullptr, nullptr, H->perm, grad);
     SUNSET_CUDA(H, cudaGetLastError());
     return 0;
 }
@@ -2118,7 +2141,7 @@ int op_laplacian(Handle *H, const double *phi, double *lap) {
     if (rc) return rc;
     StageArgs A = make_args(H, 0, 5);
     const int TB = 128, nblk = (H->nslices * kSlice + TB - 1) / TB;
-    k_op_grad_lap<<<nblk, TB, 0, H->stream>>>(A, phi, nullptr, nullptr, lap);
+    k_op_grad_lap<false><<<nblk, TB, 0, H->stream>>>(A, phi, nullptr, nullptr, lap, nullptr, nullptr);
     SUNSET_CUDA(H, cudaGetLastError());
     return 0;
 }
