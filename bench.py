@@ -619,7 +619,7 @@ def main():
                "sample": f"{k} RK steps of the full {n}-node set (weights from the device build)"}
         del o
 
-    launches_per_step = 7
+    launches_per_step = 6
     line = {"metric": METRIC, "value": value, "unit": "node-steps/s", "n_gpus": ws, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms_max / args.steps, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None, "dtype": "f64" if args.precision == "fp64" else "f32+f64",

@@ -8,7 +8,7 @@ same order, radius and form.
 Sets the workload up (neighbours, weights, link stream), sets the initial state, runs two
 graph-launched steps, then STEPS steps launched kernel by kernel through
 sunset_time_stage_kernel.  Kernel launch order after setup: the two graph steps (4 k_stage,
-1 k_filter, 1 k_finalize, 1 k_tstep each), then the STEPS direct steps in the same order, so
+1 k_filter, 1 k_finalize each), then the STEPS direct steps in the same order, so
 `-k regex:k_stage -s 9 -c 1` selects stage 1 of the first direct step and
 `-k regex:k_filter -s 2 -c 1` its filter.
 """
