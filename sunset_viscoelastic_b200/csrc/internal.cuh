@@ -205,6 +205,7 @@ struct Handle {
     // tiles of tslices slices (kTileSlices, or fewer on small sets): the sorted set of nodes their links reach (the halo) and,
     // per link, the position of its parent in that set | reflection code << 14
     int ntiles = 0, halo_max = 0, tslices = kTileSlices;
+    int nsm = 0, sm_smem = 0;  // SMs of the device, shared memory of each
     int *halo_ptr = nullptr, *halo = nullptr;
     uint16_t *lloc = nullptr;
 

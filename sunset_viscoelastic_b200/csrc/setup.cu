@@ -746,10 +746,10 @@ __global__ void __launch_bounds__(kHaloThreads) k_halo_links(int n, int nslices,
 // Two ways that keep the order gained too little: a thread a node in smaller blocks with rings
 // eight deep (4,096 nodes 96 -> 90), a warp a gathered field (95 -> 86, and 115 -> 156 at 16,384).
 static int tile_slices(Handle *H, int nslices, int *ts) {
-    int nsm = 0;
-    SUNSET_CUDA(H, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, H->device));
+    SUNSET_CUDA(H, cudaDeviceGetAttribute(&H->nsm, cudaDevAttrMultiProcessorCount, H->device));
+    SUNSET_CUDA(H, cudaDeviceGetAttribute(&H->sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, H->device));
     *ts = H->cfg.precision == SUNSET_MIXED || H->nb > 0 ? kTileSlices : 1;
-    while (*ts < kTileSlices && nslices > 2 * nsm * *ts) *ts *= 2;
+    while (*ts < kTileSlices && nslices > 2 * H->nsm * *ts) *ts *= 2;
     return 0;
 }
 

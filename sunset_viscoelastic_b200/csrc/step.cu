@@ -186,7 +186,6 @@ __device__ __forceinline__ void load_halo(const StageArgs &A, double *sm, SRC sr
 // is needed; slots are reused only after the thread has consumed them.
 template <bool MX, int NA, int D, bool SPLIT = false>
 struct LinkRing {
-    static_assert((D & (D - 1)) == 0, "ring depth must be a power of two");
     using W2 = typename std::conditional<MX, float2, double2>::type;
     W2 *w;          // [D][NA][kTile]
     unsigned *l;    // [D][kTile]
@@ -209,7 +208,7 @@ struct LinkRing {
     }
     __device__ __forceinline__ void issue(int m) {
         if (m < npair) {
-            const int s = m & (D - 1);
+            const int s = (unsigned)m % D;
             const long long o = SPLIT ? pb + m * step : pb + ((long long)m << 5);
 #pragma unroll
             for (int a = 0; a < NA; a++) cp_async_link<sizeof(W2)>(w + (s * NA + a) * kTile + threadIdx.x, src[a] + o);
@@ -227,11 +226,11 @@ struct LinkRing {
         cp_async_wait<D - 1>();
     }
     __device__ __forceinline__ void weights(int m, int a, double &x0, double &x1) const {
-        const W2 v = w[((m & (D - 1)) * NA + a) * kTile + threadIdx.x];
+        const W2 v = w[((unsigned)m % D * NA + a) * kTile + threadIdx.x];
         x0 = (double)v.x;
         x1 = (double)v.y;
     }
-    __device__ __forceinline__ unsigned index(int m) const { return l[(m & (D - 1)) * kTile + threadIdx.x]; }
+    __device__ __forceinline__ unsigned index(int m) const { return l[(unsigned)m % D * kTile + threadIdx.x]; }
 };
 
 // Ring depth: FP64 pairs are 52 bytes a thread, FP32 ones 28.
@@ -832,9 +831,9 @@ __host__ __device__ constexpr int stage_min_blocks(bool mx) { return mx ? SUNSET
 // O(dt rhs) quantity) and the error accumulator E as FP32.
 // BND: the node set has boundary nodes (walls, inflows, outflows); without them the
 // closures are compiled out, which keeps them from costing the periodic sets registers.
-template <int FORM, bool MD, bool MX, bool FP, bool BND, bool SPLIT>
+template <int FORM, bool MD, bool MX, bool FP, bool BND, bool SPLIT, int D>
 __global__ void __launch_bounds__(kTile, stage_min_blocks(MX)) k_stage(StageArgs A) {
-    static_assert(!(MX && SPLIT), "the mixed path keeps whole tiles: another order of its FP32 sums shows in the results");
+    static_assert(!((MX || BND) && SPLIT), "mixed sets and sets with boundary nodes keep whole tiles (tile_slices)");
     const StepConsts &cK = A.K;
     extern __shared__ __align__(16) double smem[];
     constexpr int NG = ngather(FORM, MD, FP);
@@ -856,7 +855,7 @@ __global__ void __launch_bounds__(kTile, stage_min_blocks(MX)) k_stage(StageArgs
         if (cK.has_mirrors) gather_stage_mx<FORM, MD, FP, true>(A, i, smem, R, active, oi, g);
         else gather_stage_mx<FORM, MD, FP, false>(A, i, smem, R, active, oi, g);
     } else {
-        LinkRing<false, 3, ring_depth(false), SPLIT> R;
+        LinkRing<false, 3, D, SPLIT> R;
         R.src[0] = reinterpret_cast<const double2 *>(A.wx);
         R.src[1] = reinterpret_cast<const double2 *>(A.wy);
         R.src[2] = reinterpret_cast<const double2 *>(A.wl);
@@ -1789,14 +1788,18 @@ constexpr size_t kMaxStageSmem = 200 * 1024;
 #define SUNSET_SMEM_ATTR(K) SUNSET_CUDA(H, cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxStageSmem))
 template <int FORM, bool MD, bool FP>
 int stage_smem_attributes(Handle *H, bool mx) {
+    constexpr int D = ring_depth(false);
     if (H->nb > 0) {
-        SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, true, false>));
-        SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, true, true>));
-        if (mx) SUNSET_SMEM_ATTR((k_stage<FORM, MD, true, FP, true, false>));
+        SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, true, false, D>));
+        SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, true, false, 3>));
+        SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, true, false, 4>));
+        if (mx) SUNSET_SMEM_ATTR((k_stage<FORM, MD, true, FP, true, false, D>));
     } else {
-        SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, false, false>));
-        SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, false, true>));
-        if (mx) SUNSET_SMEM_ATTR((k_stage<FORM, MD, true, FP, false, false>));
+        SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, false, false, D>));
+        SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, false, false, 3>));
+        SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, false, false, 4>));
+        SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, false, true, D>));
+        if (mx) SUNSET_SMEM_ATTR((k_stage<FORM, MD, true, FP, false, false, D>));
     }
     return 0;
 }
@@ -1855,23 +1858,50 @@ void launch_dependent(void (*kernel)(P...), int grid, int block, size_t smem, cu
     cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
+// The stage's link ring, in pairs, over whole FP64 tiles.  A block waits for each pair's copy in
+// turn, so where few blocks share a SM a longer ring shortens the block; where the SMs are full
+// the loads of the others fill that wait, and the longer ring only delays the halo's copies.
+// - no more tiles than SMs (sets with boundary nodes, the others split their tiles): 4 pairs.
+//   The cylinder channel (137 tiles, order 8) 0.151 -> 0.132 ms a step; 3 pairs 0.136, 6 0.133.
+// - a last wave at most half full, the longer ring costing no resident block: 3 pairs.  463 tiles
+//   (1.04 waves): order 8 362 -> 318 us (direct), 379 -> 332 (Cholesky), order 6 221 -> 207,
+//   241 -> 228; 576 (1.30): 369 -> 329, 411 -> 352, 260 -> 250, 308 -> 302; 1024 (2.31): 631 ->
+//   612, 667 -> 639, 434 -> 422, 471 -> 459; 2304 (5.19) -2 to +1 %; 4096 (9.23) 2692 -> 2663.
+// - else 2 pairs.  3 pairs took 352 tiles (0.79 waves) from 229 to 250 us, 239 -> 293, 155 -> 159,
+//   163 -> 169, 784 tiles (1.77) from 516 to 537, 536 -> 557, 317 -> 322, 344 -> 350, and where
+//   they cost a block (log-conformation order 6, 1024 tiles) 476 -> 495.
+inline int stage_ring(const Handle *H, size_t halo_bytes) {
+    constexpr int D = ring_depth(false);
+    auto bytes = [&](int d) { return halo_bytes + (size_t)d * LinkRing<false, 3, 1>::bytes(); };
+    auto blocks = [&](int d) { return std::min(stage_min_blocks(false), (int)((size_t)H->sm_smem / (bytes(d) + 1024))); };
+    if (H->ntiles <= H->nsm) return bytes(4) <= kMaxStageSmem ? 4 : bytes(3) <= kMaxStageSmem ? 3 : D;
+    const int wave = H->nsm * std::max(blocks(D), 1);
+    return blocks(3) == blocks(D) && H->ntiles > wave && (H->ntiles - 1) % wave < wave / 2 && bytes(3) <= kMaxStageSmem ? 3 : D;
+}
+
 template <int FORM, bool MD, bool FP>
 int launch_stage(Handle *H, const StageArgs &A, bool mx) {
-    const size_t smem = mx ? mx_smem_bytes(ngather(FORM, MD, FP), H->halo_max)
-                           : halo_doubles(ngather(FORM, MD, FP), H->halo_max) * sizeof(double) +
-                                 LinkRing<false, 3, ring_depth(false)>::bytes();
-    if (smem > kMaxStageSmem) return set_err(H, SUNSET_ERR_SCOPE, "tile halo too large for shared memory");
+    constexpr int D = ring_depth(false);
+    const size_t halo = mx ? 0 : halo_doubles(ngather(FORM, MD, FP), H->halo_max) * sizeof(double);
     const bool bnd = H->nb > 0, split = H->tslices < kTileSlices;
+    const int depth = mx || split ? D : stage_ring(H, halo);
+    const size_t smem = mx ? mx_smem_bytes(ngather(FORM, MD, FP), H->halo_max) : halo + depth * LinkRing<false, 3, 1>::bytes();
+    if (smem > kMaxStageSmem) return set_err(H, SUNSET_ERR_SCOPE, "tile halo too large for shared memory");
     auto go = [&](auto kernel) { launch_dependent(kernel, H->ntiles, kTile, smem, H->stream, A); };
     if (mx) {
-        if (bnd) go(k_stage<FORM, MD, true, FP, true, false>);
-        else go(k_stage<FORM, MD, true, FP, false, false>);
-    } else if (split) {
-        if (bnd) go(k_stage<FORM, MD, false, FP, true, true>);
-        else go(k_stage<FORM, MD, false, FP, false, true>);
+        if (bnd) go(k_stage<FORM, MD, true, FP, true, false, D>);
+        else go(k_stage<FORM, MD, true, FP, false, false, D>);
+    } else if (split) {  // sets without boundary nodes
+        go(k_stage<FORM, MD, false, FP, false, true, D>);
+    } else if (depth == 4) {
+        if (bnd) go(k_stage<FORM, MD, false, FP, true, false, 4>);
+        else go(k_stage<FORM, MD, false, FP, false, false, 4>);
+    } else if (depth == 3) {
+        if (bnd) go(k_stage<FORM, MD, false, FP, true, false, 3>);
+        else go(k_stage<FORM, MD, false, FP, false, false, 3>);
     } else {
-        if (bnd) go(k_stage<FORM, MD, false, FP, true, false>);
-        else go(k_stage<FORM, MD, false, FP, false, false>);
+        if (bnd) go(k_stage<FORM, MD, false, FP, true, false, D>);
+        else go(k_stage<FORM, MD, false, FP, false, false, D>);
     }
     return 0;
 }

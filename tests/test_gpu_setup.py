@@ -116,3 +116,26 @@ def test_small_set_tiles(nside, form, order):
         got = g.state()
         for k in ("ro", "u", "v", "cxx", "cxy", "cyy"):
             assert np.abs(got[k] - want[k]).max() <= tol * max(1.0, np.abs(want[k]).max()), k
+
+
+# Whole tiles on either side of a full wave (444 tiles on 148 SMs at three blocks each): 337^2
+# nodes fill it with the ring two pairs deep, 338^2 begin another with the ring three deep.  The
+# sums' rounding, eps * 20 |u| / s^2 = 5e-10, is 1e-11 of the largest right-hand side.
+@pytest.mark.parametrize("form,order", [("di", 4), ("chl", 6), ("lc", 4)])
+@pytest.mark.parametrize("nside", [337, 338])
+def test_ring_depths(nside, form, order):
+    ns = jittered_lattice(nside)
+    kw = dict(form=form, order=order, h_over_s={4: 1.5, 6: 2.1}[order])
+    O.set_pow_mode(True)
+    try:
+        ref = O.Oracle(**kw).build_domain(ns).setup()
+    finally:
+        O.set_pow_mode(False)
+    gpu = labfm.Sunset(**kw).build_domain(ns).setup()
+    st = initial_state(ns)
+    st["cxx"] = 1.3 + 0.2 * np.sin(2 * np.pi * ns.x)
+    for g in (ref, gpu):
+        g.set_state(**st)
+    a, b = gpu.rhs(), ref.rhs()
+    for k in ("ro", "rou", "rov", "xx", "xy", "yy"):
+        assert np.abs(a[k] - b[k]).max() <= 1e-10 * max(1.0, np.abs(b[k]).max()), k
