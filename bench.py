@@ -524,7 +524,7 @@ def setup_block(wl, nodes, device_s, phases):
     return {"device_s": device_s, "device_nodes_per_s": nodes / device_s, "device_phases_s": phases,
             "cpu_nodes_per_s": sns.n / el, "cpu_cores": cpu_threads(), "cpu_kind": "port",
             "cpu_sample": f"the restatement's setup of {sns.n} nodes at the same order and radius ({el:.2f} s)",
-            "note": "wall seconds through the C-ABI setup calls, host-side link ordering included"}
+            "note": "wall seconds through the C-ABI setup calls"}
 
 
 def adjoint_cost(wl, steps, checkpoint, warmup, local, reps=3):
