@@ -586,9 +586,16 @@ int sunset_calc_gradient(SunsetHandle *sh, const double *phi, double *grad, int 
     double *p = H->tmpd, *g = H->tmpd + n;
     if (int rc = to_internal(H, phi, flags, p)) return rc;
     if (int rc = op_gradient_ref(H, p, g)) return rc;
-    SUNSET_CUDA(H, cudaMemcpyAsync(grad, g, 2 * (size_t)n * sizeof(double),
-                                   flags == SUNSET_PTR_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, H->stream));
+    const size_t bytes = 2 * (size_t)n * sizeof(double);
+    if (flags != SUNSET_PTR_DEVICE) {
+        SUNSET_CUDA(H, copy_out(H, grad, g, bytes));
+        return 0;
+    }
+    // a caller's array is written on the default stream, after the work that is queued there on
+    // it (the handle's stream does not wait for that stream)
     SUNSET_CUDA(H, cudaStreamSynchronize(H->stream));
+    SUNSET_CUDA(H, cudaMemcpyAsync(grad, g, bytes, cudaMemcpyDeviceToDevice, cudaStreamLegacy));
+    SUNSET_CUDA(H, cudaStreamSynchronize(cudaStreamLegacy));
     return 0;
 }
 
