@@ -764,10 +764,13 @@ int build_halos(Handle *H) {
     int *list = nullptr, *count = nullptr, tsize = 4096, hmax = 0;
     std::vector<int> hptr(nt + 1);
     if (dalloc(H, &count, nt)) return SUNSET_ERR_NOMEM;
+    auto set_smem = [](int slots) { return (slots + slots / 2) * (int)sizeof(int); };
+    // the limit is the process's, not the handle's: always the larger set's, so that set-ups in
+    // other threads never find it too low
+    SUNSET_CUDA(H, cudaFuncSetAttribute(k_tile_halos, cudaFuncAttributeMaxDynamicSharedMemorySize, set_smem(2 * (kLocMask + 1))));
     for (;; tsize = 2 * (kLocMask + 1)) {
-        const int smem = (tsize + tsize / 2) * (int)sizeof(int);
+        const int smem = set_smem(tsize);
         if (dalloc(H, &list, (size_t)nt * (tsize / 2))) return SUNSET_ERR_NOMEM;
-        SUNSET_CUDA(H, cudaFuncSetAttribute(k_tile_halos, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         k_tile_halos<<<nt, kHaloThreads, smem, st>>>(n, nsl, H->slice_ptr, H->cnt, H->lidx, ts, tsize, list, count);
         SUNSET_CUDA(H, cudaGetLastError());
         SUNSET_CUDA(H, cudaMemcpyAsync(hptr.data() + 1, count, nt * sizeof(int), cudaMemcpyDeviceToHost, st));

@@ -1894,8 +1894,10 @@ int launch_adapt(Handle *H, AdaptArgs &a) {
     const size_t smem = (size_t)adapt_doubles<ORDER>(a.nplink) * sizeof(double);
     int optin = 0, nsm = 0, per_sm = 0;
     if (int rc = smem_optin(H, &optin)) return rc;
-    if (smem + 1024 > (size_t)optin) return set_err(H, SUNSET_ERR_SCOPE, "neighbour lists too long for the stencil adaptation");
-    SUNSET_CUDA(H, cudaFuncSetAttribute(k_adapt_stencils<ORDER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int most = optin - 1024;  // the kernel's static part beside it
+    if (smem > (size_t)most) return set_err(H, SUNSET_ERR_SCOPE, "neighbour lists too long for the stencil adaptation");
+    // the limit is the process's, so it does not follow this handle's lists (setup.cu, build_halos)
+    SUNSET_CUDA(H, cudaFuncSetAttribute(k_adapt_stencils<ORDER>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     SUNSET_CUDA(H, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, H->device));
     SUNSET_CUDA(H, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_adapt_stencils<ORDER>, T, smem));
     const int nb = std::max(1, std::min(a.w.npfb, nsm * std::max(1, per_sm)));  // each takes one node after another

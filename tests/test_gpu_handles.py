@@ -11,7 +11,7 @@ import numpy as np
 import pytest
 
 from sunset_viscoelastic_b200 import labfm
-from sunset_viscoelastic_b200.nodesets import WORKLOADS, initial_state
+from sunset_viscoelastic_b200.nodesets import WORKLOADS, initial_state, jittered_lattice
 
 pytestmark = pytest.mark.gpu
 
@@ -54,3 +54,36 @@ def test_two_configurations_from_two_threads():
             assert np.array_equal(together[key][f], alone[key][f]), (key, f)
     a.close()
     b.close()
+
+
+def test_wide_and_narrow_lists_from_two_threads():
+    """Set-ups in several threads: lists whose halos need the larger hash set in shared memory
+    (900 links a node; mixed precision keeps whole tiles) in one, ordinary ones in the others.  A
+    kernel's limit of dynamic shared memory is the process's, so no set-up may lower it between
+    another's call and launch."""
+    ns = jittered_lattice(64)
+    errors, stop = [], threading.Event()
+
+    def build(radius, n):
+        try:
+            for _ in range(n):
+                if stop.is_set():
+                    return
+                g = labfm.Sunset(form="di", order=4, h_over_s=radius / 2, precision="mixed").build_domain(ns)
+                g.find_neighbours()
+                g.close()
+        except Exception as e:  # noqa: BLE001 - reported below
+            errors.append((radius, str(e)))
+        finally:
+            if radius > 10.0:
+                stop.set()
+
+    narrow = [threading.Thread(target=build, args=(3.0, 100000)) for _ in range(3)]
+    wide = threading.Thread(target=build, args=(17.0, 600))
+    for t in narrow + [wide]:
+        t.start()
+    wide.join(120)
+    stop.set()
+    for t in narrow:
+        t.join(120)
+    assert not errors, errors[0]
