@@ -13,6 +13,11 @@
  * available from sunset_last_error().  Nothing aborts the host process.  A handle owns
  * one CUDA stream; calls on one handle must not overlap, distinct handles are independent
  * (every kernel takes its run's constants as a launch parameter).
+ *
+ * A handle takes its device memory in blocks of 4 to 64 MB, which stay with it until
+ * sunset_destroy (or until the device is out of memory, when the unused ones go back); arrays of
+ * 32 MB and more are taken and given back one by one.  A refused allocation is SUNSET_ERR_NOMEM
+ * with CUDA's answer in the message.
  */
 #ifndef SUNSET_GPU_H
 #define SUNSET_GPU_H

@@ -22,87 +22,15 @@ int set_err(Handle *H, int code, const char *fmt, ...) {
     return code;
 }
 
-// A set-up makes some 150 device arrays, and cudaMalloc and cudaFree take 0.36 and 0.30 ms each
-// however small the array is (1 MB to 128 MB alike), so the handle takes its memory in
-// blocks and cuts the arrays from them: first fit, freed neighbours joined.  A block is as
-// large as what the handle holds already, between 4 and 64 MB; an array of 32 MB and more is a
-// block of its own and is freed at once.  Nothing outlives the handle.  262,144 nodes at
-// order 6, create to close: 135 -> 87 ms; 10,000 nodes at order 8: 30 -> 14 ms.
-constexpr size_t kBlockMin = (size_t)4 << 20, kBlockMax = (size_t)64 << 20, kOwnBlock = (size_t)32 << 20;
-
-static char *new_block(size_t bytes) {
-    void *q = nullptr;
-    if (cudaMalloc(&q, bytes) == cudaSuccess) return static_cast<char *>(q);
-    cudaGetLastError();
-    return nullptr;
-}
-
-void *device_alloc(Handle *H, size_t bytes) {
-    bytes = (bytes + 255) & ~(size_t)255;
-    if (bytes < kOwnBlock) {
-        for (int pass = 0; pass < 2; pass++) {
-            for (Handle::Block &B : H->blocks)
-                for (auto it = B.free.begin(); it != B.free.end(); ++it) {
-                    if (it->second < bytes) continue;
-                    const size_t off = it->first, len = it->second;
-                    B.free.erase(it);
-                    if (len > bytes) B.free[off + bytes] = len - bytes;
-                    H->allocs[B.base + off] = bytes;
-                    return B.base + off;
-                }
-            if (pass) return nullptr;
-            size_t held = 0;
-            for (const Handle::Block &B : H->blocks) held += B.size;
-            size_t size = std::max(bytes, std::min(kBlockMax, std::max(kBlockMin, held)));
-            char *q = new_block(size);
-            if (!q) q = new_block(size = bytes);  // memory is short: no more than asked for
-            if (!q) return nullptr;
-            H->blocks.push_back({q, size, {{0, size}}});
-        }
-    }
-    char *q = new_block(bytes);
-    if (!q) return nullptr;
-    H->blocks.push_back({q, bytes, {}});
-    H->allocs[q] = bytes;
-    return q;
-}
-
-void dfree(Handle *H, void *p) {
-    if (!p) return;
-    auto it = H->allocs.find(p);
-    if (it == H->allocs.end()) return;
-    const size_t bytes = it->second;
-    H->allocs.erase(it);
-    for (size_t b = 0; b < H->blocks.size(); b++) {
-        Handle::Block &B = H->blocks[b];
-        if (p < B.base || p >= B.base + B.size) continue;
-        if (bytes == B.size && bytes >= kOwnBlock) {
-            cudaFree(p);
-            H->blocks.erase(H->blocks.begin() + b);
-            return;
-        }
-        size_t off = static_cast<char *>(p) - B.base, len = bytes;
-        auto next = B.free.lower_bound(off);
-        if (next != B.free.end() && off + len == next->first) {
-            len += next->second;
-            next = B.free.erase(next);
-        }
-        if (next != B.free.begin()) {
-            auto prev = std::prev(next);
-            if (prev->first + prev->second == off) {
-                prev->second += len;
-                return;
-            }
-        }
-        B.free[off] = len;
-        return;
-    }
-}
-
-void dfree_all(Handle *H) {
-    for (Handle::Block &B : H->blocks) cudaFree(B.base);
-    H->blocks.clear();
-    H->allocs.clear();
+DeviceBlocks device_blocks() {
+    DeviceBlocks B;
+    B.acquire = [](void **p, size_t bytes) {
+        const cudaError_t e = cudaMalloc(p, bytes);
+        if (e != cudaSuccess) cudaGetLastError();
+        return (int)e;
+    };
+    B.release = [](void *p) { cudaFree(p); };
+    return B;
 }
 
 namespace {
@@ -259,7 +187,7 @@ void sunset_destroy(SunsetHandle *sh) {
         if (H->graph[b]) cudaGraphExecDestroy(H->graph[b]);
     for (cudaGraphExec_t g : {H->adj_rec_graph, H->adj_rev_graph})
         if (g) cudaGraphExecDestroy(g);
-    dfree_all(H);
+    H->mem.clear();
     if (H->stream) cudaStreamDestroy(H->stream);
     delete sh;
 }

@@ -2,9 +2,12 @@
 // hand-written adjoint (adjoint.cuh), so the adjoint can be checked against finite
 // differences of the forward map without a GPU.  Built into libsunset_hostcheck.so; the time
 // step itself never calls it.
+#include <algorithm>
+#include <utility>
 #include <vector>
 
 #include "adjoint.cuh"
+#include "device_blocks.h"
 
 extern "C" {
 
@@ -50,6 +53,52 @@ int sunset_hostcheck_deal(int group, const uint16_t *pos, const int *small, cons
     }
     sunset::deal_slice_by_bank(group, pos, vs, vl, c_s, c, width, chosen);
     return 0;
+}
+
+// The handle's memory blocks (device_blocks.h) over a pretended device of `limit` bytes, whose
+// addresses are only numbers.  Operation k: size[k] > 0 takes that many bytes, address[k] gets the
+// piece's address (0: refused); size[k] <= 0 gives back the piece of operation -size[k].  held[k]:
+// bytes the blocks take from the device after it; calls[k]: how often the device was asked so far.
+// Returns the bytes still taken after everything is cleared, or the last refusal's error code if
+// that is 0 (42: out of memory).
+namespace {
+struct FakeDevice {
+    size_t limit, held, next;
+    int calls;
+    std::vector<std::pair<char *, size_t>> given;
+} fake;
+int fake_acquire(void **p, size_t bytes) {
+    fake.calls++;
+    if (fake.held + bytes > fake.limit) return 42;
+    *p = reinterpret_cast<char *>(fake.next);
+    fake.given.push_back({static_cast<char *>(*p), bytes});
+    fake.next += bytes + 4096;
+    fake.held += bytes;
+    return 0;
+}
+void fake_release(void *p) {
+    for (auto &g : fake.given)
+        if (g.first == p) {
+            fake.held -= g.second;
+            g.first = nullptr;
+            return;
+        }
+    fake.held = (size_t)1 << 62;  // given back twice, or never taken
+}
+}  // namespace
+int sunset_hostcheck_blocks(long long limit, int n, const long long *size, long long *address, long long *held, int *calls) {
+    fake = {(size_t)limit, 0, (size_t)1 << 40, 0, {}};
+    sunset::DeviceBlocks B;
+    B.acquire = fake_acquire;
+    B.release = fake_release;
+    for (int k = 0; k < n; k++) {
+        if (size[k] > 0) address[k] = (long long)reinterpret_cast<size_t>(B.take((size_t)size[k]));
+        else B.give(reinterpret_cast<char *>((size_t)address[-size[k]]));
+        held[k] = (long long)fake.held;
+        calls[k] = fake.calls;
+    }
+    B.clear();
+    return fake.held ? (int)std::min(fake.held, (size_t)1 << 30) : B.error;
 }
 
 // c = lc_c_from_psi(psi) and, with cbar given, psibar = cbar^T dc/dpsi.

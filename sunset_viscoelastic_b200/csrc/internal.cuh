@@ -21,11 +21,11 @@
 #include <math.h>
 #include <stdint.h>
 
-#include <map>
 #include <string>
 #include <vector>
 
 #include "../../include/sunset_gpu.h"
+#include "device_blocks.h"
 
 namespace sunset {
 
@@ -165,6 +165,8 @@ inline StepConsts step_consts(const SunsetConfig &c, int npfb, int nslices, bool
     return K;
 }
 
+DeviceBlocks device_blocks();  // of cudaMalloc and cudaFree (abi.cu)
+
 struct Handle {
     SunsetConfig cfg{};
     std::string err;
@@ -294,14 +296,7 @@ struct Handle {
     double adj_graph_dt = 0.0;                 // dt and checkpoint store the two graphs were captured with
     const double *adj_graph_cp = nullptr;
 
-    // device memory of the handle (abi.cu): blocks with their free ranges, and the pieces given out
-    struct Block {
-        char *base;
-        size_t size;
-        std::map<size_t, size_t> free;  // offset -> length
-    };
-    std::vector<Block> blocks;
-    std::map<void *, size_t> allocs;
+    DeviceBlocks mem = device_blocks();  // the handle's device memory
 };
 
 // error helpers
@@ -314,19 +309,18 @@ int set_err(Handle *H, int code, const char *fmt, ...);
                                      cudaGetErrorString(e_), __FILE__, __LINE__);               \
     } while (0)
 
-// Device memory of the handle: 256-byte aligned pieces of its blocks, null when there is none
-// left.  A freed piece may be given out again at once, so every kernel and copy that touches one
-// runs on the handle's stream (or has been waited for).
-void *device_alloc(Handle *H, size_t bytes);
+// Device memory of the handle.  A freed piece may be given out again at once, so every kernel and
+// copy that touches one runs on the handle's stream (or has been waited for).
 template <typename T>
 int dalloc(Handle *H, T **p, size_t n) {
-    void *q = device_alloc(H, (n ? n : 1) * sizeof(T));
-    if (!q) return set_err(H, SUNSET_ERR_NOMEM, "no device memory for %zu bytes", n * sizeof(T));
+    void *q = H->mem.take((n ? n : 1) * sizeof(T));
+    if (!q)
+        return set_err(H, SUNSET_ERR_NOMEM, "cudaMalloc(%zu) failed: %s", n * sizeof(T),
+                       cudaGetErrorString((cudaError_t)H->mem.error));
     *p = static_cast<T *>(q);
     return 0;
 }
-void dfree(Handle *H, void *p);
-void dfree_all(Handle *H);
+inline void dfree(Handle *H, void *p) { H->mem.give(p); }
 // device -> host on the handle's stream, waited for
 inline cudaError_t copy_out(Handle *H, void *dst, const void *src, size_t bytes) {
     cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, H->stream);

@@ -160,3 +160,19 @@ def test_call_order_and_3d_scope():
     assert code_of(g.load_checkpoint, b"\0" * 64) == labfm.ERR_ARG   # not a 3-D checkpoint of this size
     assert code_of(g.save_checkpoint) == labfm.ERR_ARG      # nothing to save before set_state_3d
     g.close()
+
+
+def test_refused_allocation_gives_the_devices_answer():
+    """An adjoint of 2e9 steps with a checkpoint each asks for 32 TB: the call returns
+    SUNSET_ERR_NOMEM with the size and what CUDA answered."""
+    wl = small("periodic-lc-o6-262k", 17)
+    ns = wl.nodes()
+    g = labfm.for_workload(wl, ns).setup()
+    st = initial_state(ns)
+    g.set_state(**st)
+    dt = wl.cfl * min(g.set_tstep())
+    with pytest.raises(labfm.SunsetError) as e:
+        g.adjoint_run(dt, 2_000_000_000, 1)
+    assert e.value.code == labfm.ERR_NOMEM
+    assert str(7 * ns.n * 2_000_000_000 * 8) in str(e.value) and "out of memory" in str(e.value)
+    g.close()
