@@ -3075,6 +3075,7 @@ int adjoint_run(Handle *H, double dt, int nsteps, int ckpt, double *J, double *d
     if (H->adj_nseg < nseg) {  // checkpoint store: grows with the number of segments
         if (H->adj_cp) dfree(H, H->adj_cp);
         H->adj_cp = nullptr;
+        H->adj_nseg = 0;
         if (dalloc(H, &H->adj_cp, (size_t)7 * n * nseg)) return SUNSET_ERR_NOMEM;
         H->adj_nseg = nseg;
     }

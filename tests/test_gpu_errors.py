@@ -176,3 +176,23 @@ def test_refused_allocation_gives_the_devices_answer():
     assert e.value.code == labfm.ERR_NOMEM
     assert str(7 * ns.n * 2_000_000_000 * 8) in str(e.value) and "out of memory" in str(e.value)
     g.close()
+
+
+def test_adjoint_after_a_refused_allocation():
+    """After an adjoint whose checkpoint store was refused, the handle runs the one it ran before."""
+    wl = small("periodic-lc-o6-262k", 17)
+    ns = wl.nodes()
+    g = labfm.for_workload(wl, ns).setup()
+    st = initial_state(ns)
+    g.set_state(**st)
+    dt = wl.cfl * min(g.set_tstep())
+    runs = []
+    for refused in (False, True):
+        if refused:
+            assert code_of(g.adjoint_run, dt, 2_000_000_000, 1) == labfm.ERR_NOMEM
+        g.set_state(**st)
+        runs.append(g.adjoint_run(dt, 3, 1))
+    (J0, p0, d0), (J1, p1, d1) = runs
+    assert J0 == J1 and p0 == p1
+    assert all(np.array_equal(d0[k], d1[k]) for k in d0)
+    g.close()
