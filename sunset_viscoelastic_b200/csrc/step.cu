@@ -20,7 +20,6 @@
 #include <algorithm>
 #include <cstring>
 #include <thread>
-#include <type_traits>
 
 #include "adjoint.cuh"
 #include "internal.cuh"
@@ -184,22 +183,21 @@ __device__ __forceinline__ void load_halo(const StageArgs &A, double *sm, SRC sr
 // indices -- D-1 pairs ahead of the pair it works on, so D-1 pairs per thread are in flight
 // without holding registers.  A thread reads back only what it copied itself, so no barrier
 // is needed; slots are reused only after the thread has consumed them.
-template <bool MX, int NA, int D, bool SPLIT = false>
+template <int NA, int D, bool SPLIT = false>
 struct LinkRing {
-    using W2 = typename std::conditional<MX, float2, double2>::type;
-    W2 *w;          // [D][NA][kTile]
+    double2 *w;     // [D][NA][kTile]
     unsigned *l;    // [D][kTile]
-    const W2 *src[NA];
+    const double2 *src[NA];
     const unsigned *lsrc;
     long long pb;   // pair index of this thread's pair 0; pair m sits at pb + 32 m (SPLIT: pb + step m)
     int npair, step;
 
-    static constexpr size_t bytes() { return (size_t)D * kTile * (NA * sizeof(W2) + sizeof(unsigned)); }
+    static constexpr size_t bytes() { return (size_t)D * kTile * (NA * sizeof(double2) + sizeof(unsigned)); }
 
     // the node's pairs start at pb_ and number npair_; the thread takes pairs part, part + parts, ...
     __device__ __forceinline__ void init(double *base, const unsigned *lidx2, long long pb_, int npair_, int part = 0,
                                          int parts = 1) {
-        w = reinterpret_cast<W2 *>(base);
+        w = reinterpret_cast<double2 *>(base);
         l = reinterpret_cast<unsigned *>(w + (size_t)D * NA * kTile);
         lsrc = lidx2;
         pb = SPLIT ? pb_ + 32 * part : pb_;
@@ -211,7 +209,7 @@ struct LinkRing {
             const int s = (unsigned)m % D;
             const long long o = SPLIT ? pb + m * step : pb + ((long long)m << 5);
 #pragma unroll
-            for (int a = 0; a < NA; a++) cp_async_link<sizeof(W2)>(w + (s * NA + a) * kTile + threadIdx.x, src[a] + o);
+            for (int a = 0; a < NA; a++) cp_async_link<sizeof(double2)>(w + (s * NA + a) * kTile + threadIdx.x, src[a] + o);
             cp_async<4>(l + s * kTile + threadIdx.x, lsrc + o);
         }
         cp_async_commit();  // empty groups keep the group count uniform
@@ -226,30 +224,19 @@ struct LinkRing {
         cp_async_wait<D - 1>();
     }
     __device__ __forceinline__ void weights(int m, int a, double &x0, double &x1) const {
-        const W2 v = w[((unsigned)m % D * NA + a) * kTile + threadIdx.x];
-        x0 = (double)v.x;
-        x1 = (double)v.y;
+        const double2 v = w[((unsigned)m % D * NA + a) * kTile + threadIdx.x];
+        x0 = v.x;
+        x1 = v.y;
     }
     __device__ __forceinline__ unsigned index(int m) const { return l[(unsigned)m % D * kTile + threadIdx.x]; }
 };
 
-// Ring depth: FP64 pairs are 52 bytes a thread, FP32 ones 28.
-#ifndef SUNSET_RING_FP64
-#define SUNSET_RING_FP64 2
-#endif
-#ifndef SUNSET_RING_MIXED
-#define SUNSET_RING_MIXED 4
-#endif
-__host__ __device__ constexpr int ring_depth(bool mx) { return mx ? SUNSET_RING_MIXED : SUNSET_RING_FP64; }
-// The filter streams one weight a link (20 bytes a thread and slot in FP64, 12 in FP32), so its
-// ring runs deeper for the same shared memory.
-#ifndef SUNSET_FILTER_RING_FP64
-#define SUNSET_FILTER_RING_FP64 4
-#endif
-#ifndef SUNSET_FILTER_RING_MIXED
-#define SUNSET_FILTER_RING_MIXED 8
-#endif
-__host__ __device__ constexpr int filter_ring_depth(bool mx) { return mx ? SUNSET_FILTER_RING_MIXED : SUNSET_FILTER_RING_FP64; }
+// Ring depth of the FP64 kernels, in pairs (52 bytes a thread and pair; the mixed ones stream their
+// links by bulk copies): where stage_ring finds no room for more, and the adjoint's.
+constexpr int kRing = 2;
+// The filter streams one weight a link (20 bytes a thread and pair), so its ring runs deeper for
+// the same shared memory.
+constexpr int kFilterRing = 4;
 
 // Doubles of the shared-memory halo, rounded up so the ring after it is 16-byte aligned.
 __host__ __device__ inline size_t halo_doubles(int ng, int hmax) { return ((size_t)ng * hmax + 1) & ~(size_t)1; }
@@ -293,10 +280,8 @@ __device__ __forceinline__ void combine_parts(const StageArgs &A, const TilePos 
 }
 
 // Stencil sums of one node over its small links, sum form of derivatives.F90:36-46,
-// neighbours read from the block's shared-memory halo.  In the mixed path the weights are
-// the FP32-rounded ones and A.gsx.. hold the FP64 sums of those, so the FP64 arithmetic
-// below evaluates the difference form sum_k w_k (phi_j - phi_i) of the rounded stencil.
-template <int FORM, bool MD, bool MX, bool FP, bool SPLIT, class RING>
+// neighbours read from the block's shared-memory halo.
+template <int FORM, bool MD, bool FP, bool SPLIT, class RING>
 __device__ __forceinline__ void gather_stage(const StageArgs &A, const TilePos &tp, const double *sm, RING &R, Grads &g) {
     const StepConsts &cK = A.K;
     const int i = tp.i, hm = A.hmax;
@@ -310,11 +295,8 @@ __device__ __forceinline__ void gather_stage(const StageArgs &A, const TilePos &
     constexpr int kFp = fp_slot(FORM, MD);
     const bool mir = cK.has_mirrors;
     const bool full = (FORM == SUNSET_FORM_DI) && cK.di_full;
-    // FP64 step: separate multiply and add, as the reference; mixed step: fused
-    auto mac = [](double &acc, double x, double w) {
-        if constexpr (MX) acc = __fma_rn(x, w, acc);
-        else acc = acc + x * w;
-    };
+    // separate multiply and add, as the reference
+    auto mac = [](double &acc, double x, double w) { acc = acc + x * w; };
     auto link = [&](int lk, double wxk, double wyk, double wlk) {
         const int j = lk & kLocMask;
         double roj = sm[j], uj = sm[hm + j], vj = sm[2 * hm + j];
@@ -856,7 +838,7 @@ __global__ void __launch_bounds__(kTile, stage_min_blocks(MX)) k_stage(StageArgs
         if (cK.has_mirrors) gather_stage_mx<FORM, MD, FP, true>(A, i, smem, R, active, oi, g);
         else gather_stage_mx<FORM, MD, FP, false>(A, i, smem, R, active, oi, g);
     } else {
-        LinkRing<false, 3, D, SPLIT> R;
+        LinkRing<3, D, SPLIT> R;
         R.src[0] = reinterpret_cast<const double2 *>(A.wx);
         R.src[1] = reinterpret_cast<const double2 *>(A.wy);
         R.src[2] = reinterpret_cast<const double2 *>(A.wl);
@@ -865,7 +847,7 @@ __global__ void __launch_bounds__(kTile, stage_min_blocks(MX)) k_stage(StageArgs
         R.prologue();  // the first link pairs stream in while the kernel before drains and the halo is staged
         dependency_wait();
         load_halo<NG>(A, smem, [&](int f) { return gather_src<FORM, MD, FP>(A.in, f); });
-        if (SPLIT || active) gather_stage<FORM, MD, false, FP, SPLIT>(A, tp, smem, R, g);
+        if (SPLIT || active) gather_stage<FORM, MD, FP, SPLIT>(A, tp, smem, R, g);
     }
     if (stage == 0 && blockIdx.x == 0 && threadIdx.x == 0) {
         A.sc->cfl_bits = 0x7ff0000000000000ull;
@@ -1063,7 +1045,7 @@ __global__ void __launch_bounds__(kTile, 4) k_filter(StageArgs A) {
     const TilePos tp = tile_pos<SPLIT>(A);
     const int i = tp.i;
     const bool live = tp.live;
-    LinkRing<false, 1, filter_ring_depth(false), SPLIT> R;
+    LinkRing<1, kFilterRing, SPLIT> R;
     R.src[0] = reinterpret_cast<const double2 *>(A.wh);
     R.init(smem + halo_doubles(nf, A.hmax), reinterpret_cast<const unsigned *>(A.lloc),
            live ? (A.slice_ptr[i >> 5] >> 1) + (i & 31) : 0, live ? A.slice_w[i >> 5] >> 1 : 0, tp.part, tp.parts);
@@ -1789,7 +1771,7 @@ constexpr size_t kMaxStageSmem = 200 * 1024;
 #define SUNSET_SMEM_ATTR(K) SUNSET_CUDA(H, cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxStageSmem))
 template <int FORM, bool MD, bool FP>
 int stage_smem_attributes(Handle *H, bool mx) {
-    constexpr int D = ring_depth(false);
+    constexpr int D = kRing;
     if (H->nb > 0) {
         SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, true, false, D>));
         SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, true, false, 3>));
@@ -1798,7 +1780,6 @@ int stage_smem_attributes(Handle *H, bool mx) {
     } else {
         SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, false, false, D>));
         SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, false, false, 3>));
-        SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, false, false, 4>));
         SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, false, true, D>));
         if (mx) SUNSET_SMEM_ATTR((k_stage<FORM, MD, true, FP, false, false, D>));
     }
@@ -1872,21 +1853,22 @@ void launch_dependent(void (*kernel)(P...), int grid, int block, size_t smem, cu
 //   163 -> 169, 784 tiles (1.77) from 516 to 537, 536 -> 557, 317 -> 322, 344 -> 350, and where
 //   they cost a block (log-conformation order 6, 1024 tiles) 476 -> 495.
 inline int stage_ring(const Handle *H, size_t halo_bytes) {
-    constexpr int D = ring_depth(false);
-    auto bytes = [&](int d) { return halo_bytes + (size_t)d * LinkRing<false, 3, 1>::bytes(); };
+    constexpr int D = kRing;
+    auto bytes = [&](int d) { return halo_bytes + (size_t)d * LinkRing<3, 1>::bytes(); };
     auto blocks = [&](int d) { return std::min(stage_min_blocks(false), (int)((size_t)H->sm_smem / (bytes(d) + 1024))); };
-    if (H->ntiles <= H->nsm) return bytes(4) <= kMaxStageSmem ? 4 : bytes(3) <= kMaxStageSmem ? 3 : D;
+    // (without boundary nodes whole tiles are always more than the SMs, tile_slices)
+    if (H->nb > 0 && H->ntiles <= H->nsm) return bytes(4) <= kMaxStageSmem ? 4 : bytes(3) <= kMaxStageSmem ? 3 : D;
     const int wave = H->nsm * std::max(blocks(D), 1);
     return blocks(3) == blocks(D) && H->ntiles > wave && (H->ntiles - 1) % wave < wave / 2 && bytes(3) <= kMaxStageSmem ? 3 : D;
 }
 
 template <int FORM, bool MD, bool FP>
 int launch_stage(Handle *H, const StageArgs &A, bool mx) {
-    constexpr int D = ring_depth(false);
+    constexpr int D = kRing;
     const size_t halo = mx ? 0 : halo_doubles(ngather(FORM, MD, FP), H->halo_max) * sizeof(double);
     const bool bnd = H->nb > 0, split = H->tslices < kTileSlices;
     const int depth = mx || split ? D : stage_ring(H, halo);
-    const size_t smem = mx ? mx_smem_bytes(ngather(FORM, MD, FP), H->halo_max) : halo + depth * LinkRing<false, 3, 1>::bytes();
+    const size_t smem = mx ? mx_smem_bytes(ngather(FORM, MD, FP), H->halo_max) : halo + depth * LinkRing<3, 1>::bytes();
     if (smem > kMaxStageSmem) return set_err(H, SUNSET_ERR_SCOPE, "tile halo too large for shared memory");
     auto go = [&](auto kernel) { launch_dependent(kernel, H->ntiles, kTile, smem, H->stream, A); };
     if (mx) {
@@ -1894,9 +1876,8 @@ int launch_stage(Handle *H, const StageArgs &A, bool mx) {
         else go(k_stage<FORM, MD, true, FP, false, false, D>);
     } else if (split) {  // sets without boundary nodes
         go(k_stage<FORM, MD, false, FP, false, true, D>);
-    } else if (depth == 4) {
-        if (bnd) go(k_stage<FORM, MD, false, FP, true, false, 4>);
-        else go(k_stage<FORM, MD, false, FP, false, false, 4>);
+    } else if (depth == 4) {  // sets with boundary nodes
+        go(k_stage<FORM, MD, false, FP, true, false, 4>);
     } else if (depth == 3) {
         if (bnd) go(k_stage<FORM, MD, false, FP, true, false, 3>);
         else go(k_stage<FORM, MD, false, FP, false, false, 3>);
@@ -1939,7 +1920,7 @@ int launch_filter(Handle *H, const StageArgs &A, bool mx) {
         }
         return 0;
     }
-    const size_t smem = halo_doubles(nf, H->halo_max) * sizeof(double) + LinkRing<false, 1, filter_ring_depth(false)>::bytes();
+    const size_t smem = halo_doubles(nf, H->halo_max) * sizeof(double) + LinkRing<1, kFilterRing>::bytes();
     if (smem > kMaxStageSmem) return set_err(H, SUNSET_ERR_SCOPE, "tile halo too large for shared memory");
     const bool split = H->tslices < kTileSlices;
     auto go = [&](auto kernel) { launch_dependent(kernel, H->ntiles, kTile, smem, H->stream, A); };
@@ -2541,10 +2522,10 @@ __device__ __forceinline__ void load_rev_halo(const RevArgs &B, T *sm, SRC src) 
 }
 
 __host__ __device__ constexpr size_t rev_stage_smem(int hmax) {
-    return (size_t)2 * kAdjPairs * hmax * sizeof(double) + LinkRing<false, 3, ring_depth(false)>::bytes();
+    return (size_t)2 * kAdjPairs * hmax * sizeof(double) + LinkRing<3, kRing>::bytes();
 }
 __host__ __device__ inline size_t rev_filter_smem(int hmax) {
-    return halo_doubles(kAdjS, hmax) * sizeof(double) + LinkRing<false, 1, ring_depth(false)>::bytes();
+    return halo_doubles(kAdjS, hmax) * sizeof(double) + LinkRing<1, kRing>::bytes();
 }
 
 // Reverse of the filter and the mass correction (rhs_lc.F90:818-893), fused with the
@@ -2559,7 +2540,7 @@ __global__ void __launch_bounds__(kTile, 2) k_adj_filter_lc(RevArgs B) {
     const int n = cK.npfb;
     const int j = blockIdx.x * kTile + threadIdx.x;
     const bool in_slice = (j >> 5) < cK.nslices;
-    LinkRing<false, 1, ring_depth(false)> R;
+    LinkRing<1, kRing> R;
     R.src[0] = reinterpret_cast<const double2 *>(B.wh);
     R.init(smem + halo_doubles(kAdjS, B.hmax), reinterpret_cast<const unsigned *>(B.locf),
            in_slice ? (B.sptr[j >> 5] >> 1) + (j & 31) : 0, in_slice ? B.sw[j >> 5] >> 1 : 0);
@@ -2625,7 +2606,7 @@ __global__ void __launch_bounds__(kTile, 2) k_adj_stage_lc(RevArgs B) {
     const int j = blockIdx.x * kTile + threadIdx.x;
     const bool in_slice = (j >> 5) < cK.nslices;
     double2 *sm = reinterpret_cast<double2 *>(smem);
-    LinkRing<false, 3, ring_depth(false)> R;
+    LinkRing<3, kRing> R;
     R.src[0] = reinterpret_cast<const double2 *>(B.wx);
     R.src[1] = reinterpret_cast<const double2 *>(B.wy);
     R.src[2] = reinterpret_cast<const double2 *>(B.wl);
