@@ -192,7 +192,7 @@ struct LinkRing {
     long long pb;   // pair index of this thread's pair 0; pair m sits at pb + 32 m (SPLIT: pb + step m)
     int npair, step;
 
-    static constexpr size_t bytes() { return (size_t)D * kTile * (NA * sizeof(double2) + sizeof(unsigned)); }
+    __host__ __device__ static constexpr size_t bytes() { return (size_t)D * kTile * (NA * sizeof(double2) + sizeof(unsigned)); }
 
     // the node's pairs start at pb_ and number npair_; the thread takes pairs part, part + parts, ...
     __device__ __forceinline__ void init(double *base, const unsigned *lidx2, long long pb_, int npair_, int part = 0,
@@ -258,9 +258,11 @@ __device__ __forceinline__ TilePos tile_pos(const StageArgs &A) {
     p.live = p.slice < A.K.nslices;
     return p;
 }
+// Scratch of combine_parts a sum: the values of half the block.
+__host__ __device__ constexpr size_t combine_bytes() { return kTile / 2 * sizeof(double); }
 // Adds the parts' sums into part 0's, halving the parts each time; each(fn) applies fn to every
-// sum of the thread.  All threads of the block take part.  buf holds 128 values a sum: it is the
-// link ring's space, which no thread reads any more.
+// sum of the thread.  All threads of the block take part.  buf holds combine_bytes() a sum: it is
+// the link ring's space, which no thread reads any more.
 template <class EACH>
 __device__ __forceinline__ void combine_parts(const StageArgs &A, const TilePos &tp, double *buf, EACH each) {
     const int part = tp.part;
@@ -279,6 +281,12 @@ __device__ __forceinline__ void combine_parts(const StageArgs &A, const TilePos 
     }
 }
 
+// Sums of a node in gather_stage.
+__host__ __device__ constexpr int nsums(int form, bool md, bool fp) {
+    const bool di = form == SUNSET_FORM_DI, lc = form == SUNSET_FORM_LC, chl = form == SUNSET_FORM_CHL;
+    return 8 + (di || lc ? 4 : 0) + (di ? 2 : 0) + (lc || chl ? 6 : 0) + (md && (di || chl) ? 3 : 0) +
+           (fp && form != SUNSET_FORM_NEWT ? 3 : 0);
+}
 // Stencil sums of one node over its small links, sum form of derivatives.F90:36-46,
 // neighbours read from the block's shared-memory halo.
 template <int FORM, bool MD, bool FP, bool SPLIT, class RING>
@@ -364,6 +372,7 @@ __device__ __forceinline__ void gather_stage(const StageArgs &A, const TilePos &
         link((int)(l2 >> 16), wx1, wy1, wl1);
     }
     if constexpr (SPLIT) {
+        static_assert(nsums(FORM, MD, FP) * combine_bytes() <= RING::bytes(), "the parts' sums are combined in the ring's space");
         combine_parts(A, tp, reinterpret_cast<double *>(R.w), [&](auto f) {
             f(s_ro_x); f(s_ro_y); f(s_u_x); f(s_u_y); f(s_lu); f(s_v_x); f(s_v_y); f(s_lv);
             if constexpr (FORM == SUNSET_FORM_DI || FORM == SUNSET_FORM_LC) {
@@ -1089,11 +1098,13 @@ __global__ void __launch_bounds__(kTile, 4) k_filter(StageArgs A) {
             link((int)(l2 & 0xffffu), wh0);
             link((int)(l2 >> 16), wh1);
         }
-        if constexpr (SPLIT)
+        if constexpr (SPLIT) {
+            static_assert(nf * combine_bytes() <= decltype(R)::bytes(), "the parts' sums are combined in the ring's space");
             combine_parts(A, tp, reinterpret_cast<double *>(R.w), [&](auto f) {
 #pragma unroll
                 for (int q = 0; q < nf; q++) f(t[q]);
             });
+        }
         if (i < cK.npfb && (!SPLIT || tp.part == 0)) {
             const double hs = A.hsum[i];
             const double *src[7] = {F.ro, F.rou, F.rov, F.q[0], F.q[1], F.q[2], F.q[3]};
@@ -1715,7 +1726,6 @@ StepConsts consts_of(const Handle *H) {
 }
 
 StageArgs make_args(Handle *H, int from, int stage, bool step = false) {
-    const bool mx = step && H->cfg.precision == SUNSET_MIXED;
     StageArgs A{};
     A.K = consts_of(H);
     A.slice_ptr = H->slice_ptr;
