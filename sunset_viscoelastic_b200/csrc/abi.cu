@@ -1080,4 +1080,13 @@ int sunset_time_stage_kernel(SunsetHandle *sh, int reps, double *ms_per_launch, 
     return time_stage_kernel(H, reps, ms_per_launch, bytes_per_launch);
 }
 
+// What the time step's kernels run on, for the tests that aim at one route (not part of the
+// interface in include/sunset_gpu.h): slices a tile, tiles, largest halo, pairs in the stage's ring.
+int sunset_check_tiles(SunsetHandle *sh, int *out) {
+    if (!sh || !out) return SUNSET_ERR_ARG;
+    if (int rc = need(&sh->H, sh->H.nbr_ok, "sunset_find_neighbours")) return rc;
+    step_tiles(&sh->H, out);
+    return 0;
+}
+
 }  // extern "C"

@@ -387,6 +387,7 @@ int op_gradient_ref(Handle *H, const double *phi, double *grad);  // reference o
 int op_laplacian(Handle *H, const double *phi, double *lap);
 int op_filter(Handle *H, const double *phi, double *out, int term_only);
 int reduce_ke_mass(Handle *H, double *ke, double *mass);
+void step_tiles(const Handle *H, int *out);  // slices a tile, tiles, largest halo, pairs in the stage's ring
 // Field dumps and checkpoints (step.cu)
 int dump_columns(Handle *H, double *out);  // 10 x npfb, internal order, on the device
 size_t checkpoint_bytes(const Handle *H);
