@@ -11,6 +11,9 @@ the Cholesky form with both options leave; 447 tiles (338^2) begin a second wave
 The sums' rounding, eps * 20 |u| / s^2 = 5e-10 in the viscous terms, is 1e-11 of the largest
 right-hand side; 1e-10 of it is allowed, as in the set-up's tests.
 
+The same for channels with walls, which keep whole tiles at every size: the ring is four pairs deep
+up to one tile a SM (the other walled tests), two pairs above, three as without walls.
+
 And the tile halos of a stencil that reaches more than 2048 nodes from a tile, where the hash set
 that gathers them takes its larger size (mixed precision keeps whole tiles on small sets)."""
 import ctypes as C
@@ -20,7 +23,7 @@ import numpy as np
 import pytest
 
 from sunset_viscoelastic_b200 import labfm
-from sunset_viscoelastic_b200.nodesets import initial_state, jittered_lattice
+from sunset_viscoelastic_b200.nodesets import channel, initial_state, jittered_lattice, poiseuille_state
 import oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -95,6 +98,49 @@ def test_whole_tiles(form, options, nside, radius, ring):
 def test_whole_tiles_symmetric(form, ring):
     ns = dataclasses.replace(jittered_lattice(276), bcond=(1, 1, 2, 2))
     check(ns, form, dict(order=4, h_over_s=1.5), ring)
+
+
+# form, order, cells across, options, pairs in the ring: 158, 308 and 453 tiles on 148 SMs
+WALLS = [("di", 6, 200, {}, 2), ("chl", 6, 200, {}, 2), ("lc", 6, 200, {}, 2), ("di", 6, 200, MDIFF, 2), ("chl", 6, 200, FENEP, 2),
+         ("di", 4, 340, {}, 3), ("chl", 4, 340, {}, 3), ("lc", 6, 280, {}, 3), ("lc", 6, 280, FENEP, 3), ("newt", 4, 340, {}, 3)]
+
+
+@pytest.mark.parametrize("form,order,ny,options,ring", WALLS,
+                         ids=[f"{f}-o{o}-{n}{'-fenep' if 'fenep' in k else ''}{'-mdiff' if 'Mdiff' in k else ''}"
+                              for f, o, n, k, _ in WALLS])
+def test_walled_tiles(form, order, ny, options, ring):
+    grav = 8.0
+    ns = channel(ny)
+    ref, gpu = pair(ns, form=form, order=order, Re=1.0, Wi=0.5, beta=0.59, Ma=0.1, grav=(grav, 0.0, 0.0),
+                    kolmogorov_forcing=0, **options)
+    route = tiles(gpu)
+    assert route[0] == 8 and route[1] > 148 and route[3] == ring, route
+    nd, npfb = ref.nodes(), ref.sizes()[1]
+    x, y, t = nd["x"][:npfb], nd["y"][:npfb], nd["node_type"][:npfb]
+    st = poiseuille_state(type("P", (), {"y": y, "n": npfb}), grav, 1.0, 0.5)
+    st["u"] = st["u"] + 0.3 * np.sin(2 * np.pi * x) * y * (1.0 - y)
+    st["v"] = 0.2 * np.cos(2 * np.pi * x) * y * (1.0 - y)
+    st["ro"] = 1.0 + 0.01 * np.sin(2 * np.pi * x) * np.cos(np.pi * y)
+    st["cxx"] = st["cxx"] + 0.1 * np.sin(2 * np.pi * x) ** 2
+    st["cyy"] = st["cyy"] + 0.05 * np.cos(np.pi * y) ** 2
+    for g in (ref, gpu):
+        g.set_state(**st)
+    a, b = gpu.rhs(), ref.rhs()
+    # 1e-10 of the terms, as on the small channels, and eight roundings of the viscous sums, whose
+    # terms are 20 |u| / s^2 (the weights of the rows next to walls agree to rounding only)
+    gu = np.abs(ref.gradient(st["u"])).max()
+    scale = max(gu, *(np.abs(b[k]).max() for k in ("rou", "rov"))) * max(1.0, *(np.abs(st[k]).max() for k in ("cxx", "cyy")))
+    bound = 1e-10 * scale + 8 * 2.2e-16 * 20 * ny * ny
+    for k in b:
+        assert np.abs(a[k] - b[k]).max() <= bound, k
+    dt = 0.3 * min(ref.set_tstep())
+    for g in (ref, gpu):
+        g.step(dt, 3)
+    a, b = gpu.state(), ref.state()
+    for k in ("ro", "u", "v") + (() if form == "newt" else ("cxx", "cxy", "cyy")):
+        assert np.abs(a[k] - b[k]).max() <= 1e-10 * max(1.0, np.abs(b[k]).max()), k
+    assert np.all(a["rou"][t == 0] == 0.0)
+    gpu.close()
 
 
 def test_halos_of_more_than_2048_nodes():
