@@ -312,27 +312,37 @@ int make_stream_links(Handle *H) {
 }  // namespace sunset
 
 // The device's link order on host arrays in the SELL layout, for the test that compares it with
-// deal_slice_by_bank (not part of the interface in include/sunset_gpu.h).
-extern "C" int sunset_check_deal(int group, int nslices, const long long *slice_ptr, const int *slice_w, const int *cnt,
-                                 const int *cnt_small, const uint16_t *pos, int width, int *src) {
+// deal_slice_by_bank at both group sizes (not part of the interface in include/sunset_gpu.h).
+static int check_deal(sunset::Handle *H, int group, int nslices, const long long *slice_ptr, const int *slice_w, const int *cnt,
+                      const int *cnt_small, const uint16_t *pos, int width, int *src) {
     using namespace sunset;
-    Handle H;
     const int n = nslices * kSlice;
     const size_t L = (size_t)slice_ptr[nslices];
     long long *dp;
     int *dw, *dc, *ds, *dsrc;
     uint16_t *dpos;
-    int rc = SUNSET_ERR_NOMEM;
-    if (!dalloc(&H, &dp, nslices + 1) && !dalloc(&H, &dw, nslices) && !dalloc(&H, &dc, n) && !dalloc(&H, &ds, n) &&
-        !dalloc(&H, &dpos, L) && !dalloc(&H, &dsrc, L)) {
-        cudaMemcpy(dp, slice_ptr, (nslices + 1) * sizeof(long long), cudaMemcpyHostToDevice);
-        cudaMemcpy(dw, slice_w, nslices * sizeof(int), cudaMemcpyHostToDevice);
-        cudaMemcpy(dc, cnt, n * sizeof(int), cudaMemcpyHostToDevice);
-        cudaMemcpy(ds, cnt_small, n * sizeof(int), cudaMemcpyHostToDevice);
-        cudaMemcpy(dpos, pos, L * sizeof(uint16_t), cudaMemcpyHostToDevice);
-        cudaDeviceSynchronize();
-        rc = deal_links(&H, group, n, nslices, dp, dw, dc, ds, dpos, width, dsrc);
-        if (!rc && cudaMemcpy(src, dsrc, L * sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) rc = SUNSET_ERR_CUDA;
+    if (dalloc(H, &dp, nslices + 1) || dalloc(H, &dw, nslices) || dalloc(H, &dc, n) || dalloc(H, &ds, n) || dalloc(H, &dpos, L) ||
+        dalloc(H, &dsrc, L))
+        return SUNSET_ERR_NOMEM;
+    SUNSET_CUDA(H, cudaMemcpyAsync(dp, slice_ptr, (nslices + 1) * sizeof(long long), cudaMemcpyHostToDevice, H->stream));
+    SUNSET_CUDA(H, cudaMemcpyAsync(dw, slice_w, nslices * sizeof(int), cudaMemcpyHostToDevice, H->stream));
+    SUNSET_CUDA(H, cudaMemcpyAsync(dc, cnt, n * sizeof(int), cudaMemcpyHostToDevice, H->stream));
+    SUNSET_CUDA(H, cudaMemcpyAsync(ds, cnt_small, n * sizeof(int), cudaMemcpyHostToDevice, H->stream));
+    SUNSET_CUDA(H, cudaMemcpyAsync(dpos, pos, L * sizeof(uint16_t), cudaMemcpyHostToDevice, H->stream));
+    if (int rc = deal_links(H, group, n, nslices, dp, dw, dc, ds, dpos, width, dsrc)) return rc;
+    SUNSET_CUDA(H, copy_out(H, src, dsrc, L * sizeof(int)));
+    return 0;
+}
+
+extern "C" int sunset_check_deal(int group, int nslices, const long long *slice_ptr, const int *slice_w, const int *cnt,
+                                 const int *cnt_small, const uint16_t *pos, int width, int *src) {
+    if (group != 8 && group != 16) return SUNSET_ERR_ARG;
+    sunset::Handle H;
+    int rc = SUNSET_ERR_CUDA;
+    if (cudaStreamCreateWithFlags(&H.stream, cudaStreamNonBlocking) == cudaSuccess) {
+        rc = check_deal(&H, group, nslices, slice_ptr, slice_w, cnt, cnt_small, pos, width, src);
+        cudaStreamSynchronize(H.stream);
+        cudaStreamDestroy(H.stream);
     }
     H.mem.clear();
     return rc;

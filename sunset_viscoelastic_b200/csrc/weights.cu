@@ -1794,9 +1794,8 @@ __global__ void __launch_bounds__(bidiag_threads(ORDER), adapt_blocks(ORDER)) k_
     }
 }
 
-// The largest dynamic shared memory a block may opt into on the handle's device (227 KB on
-// B200): the weight and adaptation kernels are latency-bound, one warp a node, so as many
-// warps as their per-warp matrices fit.
+// The largest dynamic shared memory a block may opt into on the handle's device (227 KB on B200):
+// longer neighbour lists than fit there are refused by the adaptation.
 int smem_optin(Handle *H, int *bytes) {
     SUNSET_CUDA(H, cudaDeviceGetAttribute(bytes, cudaDevAttrMaxSharedMemoryPerBlockOptin, H->device));
     return 0;
