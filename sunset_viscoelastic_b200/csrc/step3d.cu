@@ -161,7 +161,11 @@ __host__ __device__ constexpr FDesc desc3f(int d) {
 //   Cholesky and log-conformation (10 to 16 fields): 2 links, 4 blocks, with the next links' indices
 //   fetched a batch ahead so that the field loads do not wait for them.  Cholesky at order 6, 90^2 x
 //   65 1.99 -> 1.81 ms; log-conformation at order 6, 96^2 x 65 3.00 -> 2.95 (4 links 2.93 and 3
-//   blocks 2.87 there, but 0.31 -> 0.36 at 50^2 x 30); the direct form loses by it (2.90).
+//   blocks 2.87 there, but 0.31 -> 0.36 at 50^2 x 30); the direct form loses by it (2.90).  Not on
+//   sets with mirrors (48^2 x 49, order 6: log-conformation 523 -> 541 us, Cholesky 394 -> 399,
+//   with FENE-P 415 -> 423) nor in the log-conformation form beside boundary nodes (inflow 591 ->
+//   611, walls 545 -> 537): their signs and branches take the registers it needs.  Cholesky beside
+//   walls 402 -> 357 us, the Newtonian form everywhere 9 to 14 %.
 #ifndef SUNSET_3D_BLOCKS
 #define SUNSET_3D_BLOCKS 4
 #endif
@@ -176,7 +180,8 @@ template <int FORM, bool MD, bool FULL, bool FEN, bool BND, bool MIR, class ST>
 __device__ __forceinline__ void derivs3_body(const Layer3 &L, const Fields3 &F, const ZThread &z, ST store) {
     constexpr int N = ndesc3<FORM, MD, FEN>();
     constexpr int LB = links_in_flight(FORM);
-    constexpr bool AHEAD = LB == 2;  // fetch the next links' indices a batch ahead
+    // fetch the next links' indices a batch ahead
+    constexpr bool AHEAD = LB == 2 && (FORM == SUNSET_FORM_NEWT || !MIR || (BND && FORM == SUNSET_FORM_CHL));
     constexpr bool kCL = BND && MD;
     const int k = z.k, i = z.i, iz = z.iz, row = i * L.nz, h = L.ncfd / 2;
     double sx[N], sy[N], sl[N];
