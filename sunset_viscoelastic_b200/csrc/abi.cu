@@ -1084,7 +1084,7 @@ int sunset_time_stage_kernel(SunsetHandle *sh, int reps, double *ms_per_launch, 
 // interface in include/sunset_gpu.h): slices a tile, tiles, largest halo, pairs in the stage's ring.
 int sunset_check_tiles(SunsetHandle *sh, int *out) {
     if (!sh || !out) return SUNSET_ERR_ARG;
-    if (int rc = need(&sh->H, sh->H.nbr_ok, "sunset_find_neighbours")) return rc;
+    if (int rc = need(&sh->H, sh->H.fc_ok, "sunset_filter_coefficients")) return rc;  // (sets the kernels' limits)
     step_tiles(&sh->H, out);
     return 0;
 }

@@ -1779,17 +1779,24 @@ int upload_consts(Handle *) { return 0; }
 constexpr size_t kMaxStageSmem = 200 * 1024;
 
 #define SUNSET_SMEM_ATTR(K) SUNSET_CUDA(H, cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxStageSmem))
+// The variants that stage_ring (below) gives rings of three and of four pairs, the latter with
+// boundary nodes only.
+__host__ __device__ constexpr bool ring_of_three(int form, bool md, bool fp, bool bnd) {
+    return !(fp && (ngather(form, md, fp) > 9 || (bnd && md)));
+}
+__host__ __device__ constexpr bool ring_of_four(int form, bool md, bool fp) { return !(form == SUNSET_FORM_DI && md && fp); }
+
 template <int FORM, bool MD, bool FP>
 int stage_smem_attributes(Handle *H, bool mx) {
     constexpr int D = kRing;
     if (H->nb > 0) {
         SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, true, false, D>));
-        SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, true, false, 3>));
-        SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, true, false, 4>));
+        if constexpr (ring_of_three(FORM, MD, FP, true)) SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, true, false, 3>));
+        if constexpr (ring_of_four(FORM, MD, FP)) SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, true, false, 4>));
         if (mx) SUNSET_SMEM_ATTR((k_stage<FORM, MD, true, FP, true, false, D>));
     } else {
         SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, false, false, D>));
-        SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, false, false, 3>));
+        if constexpr (ring_of_three(FORM, MD, FP, false)) SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, false, false, 3>));
         SUNSET_SMEM_ATTR((k_stage<FORM, MD, false, FP, false, true, D>));
         if (mx) SUNSET_SMEM_ATTR((k_stage<FORM, MD, true, FP, false, false, D>));
     }
@@ -1853,23 +1860,59 @@ void launch_dependent(void (*kernel)(P...), int grid, int block, size_t smem, cu
 // The stage's link ring, in pairs, over whole FP64 tiles.  A block waits for each pair's copy in
 // turn, so where few blocks share a SM a longer ring shortens the block; where the SMs are full
 // the loads of the others fill that wait, and the longer ring only delays the halo's copies.
-// - no more tiles than SMs (sets with boundary nodes, the others split their tiles): 4 pairs.
+// - no more tiles than SMs (sets with boundary nodes, the others split their tiles): 4 pairs, with
+//   up to seven gathered fields at every size (0.99 to 1.22 of the two-pair ring's rate; 12 % more on
+//   average between half a tile and one a SM).  With more fields the halo's copies weigh more and
+//   tiny sets lose by it (log-conformation, 11 tiles 100 -> 105 us, Cholesky with diffusion 113 ->
+//   118), so only above half a tile a SM (132 tiles, order 8: 144 -> 129).  With FENE-P beside them
+//   long lists decide: Cholesky with diffusion at any size at orders 6 and 8 (2 to 13 %; order 4
+//   119 -> 132), log-conformation above half a tile a SM at those orders (4 to 8 %; order 4
+//   98 -> 105); the direct form with both keeps two pairs (106 -> 117).
 //   The cylinder channel (137 tiles, order 8) 0.151 -> 0.132 ms a step; 3 pairs 0.136, 6 0.133.
 // - a last wave at most half full, the longer ring costing no resident block: 3 pairs.  463 tiles
 //   (1.04 waves): order 8 362 -> 318 us (direct), 379 -> 332 (Cholesky), order 6 221 -> 207,
 //   241 -> 228; 576 (1.30): 369 -> 329, 411 -> 352, 260 -> 250, 308 -> 302; 1024 (2.31): 631 ->
 //   612, 667 -> 639, 434 -> 422, 471 -> 459; 2304 (5.19) -2 to +1 %; 4096 (9.23) 2692 -> 2663.
+//   The resident blocks are asked for, since they depend on registers and static shared memory
+//   too: the Newtonian form has four (447 and 535 tiles are its first wave: 154 -> 166, 170 ->
+//   202), of which it may give one up for the same number of waves (625 tiles 230 -> 212); FENE-P
+//   with seven fields loses its third to 256 bytes at 1024 tiles of order 8 (694 -> 715).
+// - not with FENE-P and ten or eleven gathered fields (log-conformation, Cholesky with diffusion),
+//   nor in the direct form with both beside boundary nodes, whose kernels spill more with three
+//   pairs: 235 -> 277 us, 268 -> 280, 297 -> 310, slower at 40 of 42 sizes up to 900^2 nodes.
 // - else 2 pairs.  3 pairs took 352 tiles (0.79 waves) from 229 to 250 us, 239 -> 293, 155 -> 159,
 //   163 -> 169, 784 tiles (1.77) from 516 to 537, 536 -> 557, 317 -> 322, 344 -> 350, and where
 //   they cost a block (log-conformation order 6, 1024 tiles) 476 -> 495.
-inline int stage_ring(const Handle *H, size_t halo_bytes) {
-    constexpr int D = kRing;
-    auto bytes = [&](int d) { return halo_bytes + (size_t)d * LinkRing<3, 1>::bytes(); };
-    auto blocks = [&](int d) { return std::min(stage_min_blocks(false), (int)((size_t)H->sm_smem / (bytes(d) + 1024))); };
+constexpr int kLongLists = 64;  // link slots a node: orders 6 and 8 at the reference's radii have 72 and 92 links, order 4 41
+template <int FORM, bool MD, bool FP, bool BND>
+int stage_ring(const Handle *H) {
+    constexpr int D = kRing, NG = ngather(FORM, MD, FP);
+    const size_t halo = halo_doubles(NG, H->halo_max) * sizeof(double);
+    auto bytes = [&](int d) { return halo + (size_t)d * LinkRing<3, 1>::bytes(); };
     // (without boundary nodes whole tiles are always more than the SMs, tile_slices)
-    if (H->nb > 0 && H->ntiles <= H->nsm) return bytes(4) <= kMaxStageSmem ? 4 : bytes(3) <= kMaxStageSmem ? 3 : D;
-    const int wave = H->nsm * std::max(blocks(D), 1);
-    return blocks(3) == blocks(D) && H->ntiles > wave && (H->ntiles - 1) % wave < wave / 2 && bytes(3) <= kMaxStageSmem ? 3 : D;
+    if (BND && H->ntiles <= H->nsm) {
+        const bool wide = 2 * H->ntiles > H->nsm, lists = H->nlinks_sell > (long long)kLongLists * H->npfb;
+        const bool four = NG <= 7 || (!FP && wide) || (FP && lists && (FORM == SUNSET_FORM_CHL || (FORM == SUNSET_FORM_LC && wide)));
+        return ring_of_four(FORM, MD, FP) && four && bytes(4) <= kMaxStageSmem ? 4 : D;
+    }
+    if constexpr (ring_of_three(FORM, MD, FP, BND)) {
+        if (bytes(3) > kMaxStageSmem) return D;
+        auto resident = [&](auto kernel, int d) {
+            int n = 0;
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kTile, bytes(d));
+            return std::max(n, 1);
+        };
+        const int two = resident(k_stage<FORM, MD, false, FP, BND, false, D>, D);
+        const int three = resident(k_stage<FORM, MD, false, FP, BND, false, 3>, 3);
+        const int wave = H->nsm * two, wave3 = H->nsm * three;
+        const bool keeps = three == two || (three >= 3 && (H->ntiles - 1) / wave3 == (H->ntiles - 1) / wave);
+        if (keeps && H->ntiles > wave && (H->ntiles - 1) % wave < wave / 2) return 3;
+    }
+    return D;
+}
+template <int FORM, bool MD, bool FP>
+int stage_ring(const Handle *H) {
+    return H->nb > 0 ? stage_ring<FORM, MD, FP, true>(H) : stage_ring<FORM, MD, FP, false>(H);
 }
 
 template <int FORM, bool MD, bool FP>
@@ -1877,7 +1920,7 @@ int launch_stage(Handle *H, const StageArgs &A, bool mx) {
     constexpr int D = kRing;
     const size_t halo = mx ? 0 : halo_doubles(ngather(FORM, MD, FP), H->halo_max) * sizeof(double);
     const bool bnd = H->nb > 0, split = H->tslices < kTileSlices;
-    const int depth = mx || split ? D : stage_ring(H, halo);
+    const int depth = mx || split ? D : stage_ring<FORM, MD, FP>(H);
     const size_t smem = mx ? mx_smem_bytes(ngather(FORM, MD, FP), H->halo_max) : halo + depth * LinkRing<3, 1>::bytes();
     if (smem > kMaxStageSmem) return set_err(H, SUNSET_ERR_SCOPE, "tile halo too large for shared memory");
     auto go = [&](auto kernel) { launch_dependent(kernel, H->ntiles, kTile, smem, H->stream, A); };
@@ -1887,10 +1930,11 @@ int launch_stage(Handle *H, const StageArgs &A, bool mx) {
     } else if (split) {  // sets without boundary nodes
         go(k_stage<FORM, MD, false, FP, false, true, D>);
     } else if (depth == 4) {  // sets with boundary nodes
-        go(k_stage<FORM, MD, false, FP, true, false, 4>);
+        if constexpr (ring_of_four(FORM, MD, FP)) go(k_stage<FORM, MD, false, FP, true, false, 4>);
+    } else if (depth == 3 && bnd) {
+        if constexpr (ring_of_three(FORM, MD, FP, true)) go(k_stage<FORM, MD, false, FP, true, false, 3>);
     } else if (depth == 3) {
-        if (bnd) go(k_stage<FORM, MD, false, FP, true, false, 3>);
-        else go(k_stage<FORM, MD, false, FP, false, false, 3>);
+        if constexpr (ring_of_three(FORM, MD, FP, false)) go(k_stage<FORM, MD, false, FP, false, false, 3>);
     } else {
         if (bnd) go(k_stage<FORM, MD, false, FP, true, false, D>);
         else go(k_stage<FORM, MD, false, FP, false, false, D>);
@@ -1898,20 +1942,32 @@ int launch_stage(Handle *H, const StageArgs &A, bool mx) {
     return 0;
 }
 
-// A must come from make_args(..., step = true); mx is the handle's precision.
-int launch_stage_any(Handle *H, const StageArgs &A, bool mx) {
+// f(variant) for the handle's form and options: the variant's FORM, MD (polymer diffusion) and FP
+// (FENE-P) as compile-time constants.
+template <int F, bool M, bool P>
+struct StageVariant {
+    static constexpr int FORM = F;
+    static constexpr bool MD = M, FP = P;
+};
+template <class FN>
+int with_variant(const Handle *H, FN f) {
     const bool md = H->cfg.Mdiff != 0.0, fp = H->cfg.fenep != 0;
     switch (H->cfg.form) {
     case SUNSET_FORM_DI:
-        if (md) return fp ? launch_stage<SUNSET_FORM_DI, true, true>(H, A, mx) : launch_stage<SUNSET_FORM_DI, true, false>(H, A, mx);
-        return fp ? launch_stage<SUNSET_FORM_DI, false, true>(H, A, mx) : launch_stage<SUNSET_FORM_DI, false, false>(H, A, mx);
+        if (md) return fp ? f(StageVariant<SUNSET_FORM_DI, true, true>{}) : f(StageVariant<SUNSET_FORM_DI, true, false>{});
+        return fp ? f(StageVariant<SUNSET_FORM_DI, false, true>{}) : f(StageVariant<SUNSET_FORM_DI, false, false>{});
     case SUNSET_FORM_CHL:
-        if (md) return fp ? launch_stage<SUNSET_FORM_CHL, true, true>(H, A, mx) : launch_stage<SUNSET_FORM_CHL, true, false>(H, A, mx);
-        return fp ? launch_stage<SUNSET_FORM_CHL, false, true>(H, A, mx) : launch_stage<SUNSET_FORM_CHL, false, false>(H, A, mx);
+        if (md) return fp ? f(StageVariant<SUNSET_FORM_CHL, true, true>{}) : f(StageVariant<SUNSET_FORM_CHL, true, false>{});
+        return fp ? f(StageVariant<SUNSET_FORM_CHL, false, true>{}) : f(StageVariant<SUNSET_FORM_CHL, false, false>{});
     case SUNSET_FORM_LC:
-        return fp ? launch_stage<SUNSET_FORM_LC, false, true>(H, A, mx) : launch_stage<SUNSET_FORM_LC, false, false>(H, A, mx);
-    default: return launch_stage<SUNSET_FORM_NEWT, false, false>(H, A, mx);
+        return fp ? f(StageVariant<SUNSET_FORM_LC, false, true>{}) : f(StageVariant<SUNSET_FORM_LC, false, false>{});
+    default: return f(StageVariant<SUNSET_FORM_NEWT, false, false>{});
     }
+}
+
+// A must come from make_args(..., step = true); mx is the handle's precision.
+int launch_stage_any(Handle *H, const StageArgs &A, bool mx) {
+    return with_variant(H, [&](auto v) { return launch_stage<decltype(v)::FORM, decltype(v)::MD, decltype(v)::FP>(H, A, mx); });
 }
 
 template <int FORM>
@@ -2194,12 +2250,12 @@ int reduce_ke_mass(Handle *H, double *ke, double *mass) {
 
 // What the FP64 time step runs on: slices a tile, tiles, largest halo, pairs in the stage's ring.
 void step_tiles(const Handle *H, int *out) {
-    const bool fp = H->cfg.fenep != 0, split = H->tslices < kTileSlices;
-    const size_t halo = halo_doubles(ngather(H->cfg.form, H->cfg.Mdiff != 0.0, fp), H->halo_max) * sizeof(double);
     out[0] = H->tslices;
     out[1] = H->ntiles;
     out[2] = H->halo_max;
-    out[3] = is_mx(H) || split ? kRing : stage_ring(H, halo);
+    out[3] = kRing;
+    if (!is_mx(H) && H->tslices == kTileSlices)
+        out[3] = with_variant(H, [&](auto v) { return stage_ring<decltype(v)::FORM, decltype(v)::MD, decltype(v)::FP>(H); });
 }
 
 // Average duration of the RK stage kernel inside real steps: `reps` steps at the current dt
